@@ -17,7 +17,7 @@ OUT_DIR = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT_DIR, "libgbpt.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["kernels_wave.cu", "kernels_adapt.cu", "api.cu", "noalloc.cu", "image.cu", "texture.cu", "mlp.cu",
-           "bvh_build.cpp", "server.cpp"]
+           "bvh_build.cpp", "ordered_tree.cpp", "server.cpp"]
 
 
 def _nvcc():

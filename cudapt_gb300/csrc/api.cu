@@ -86,7 +86,8 @@ struct gbpt_scene {
     uint32_t w = 0, h = 0;
   };
   std::vector<Texture> textures;  // RTScene::m_pTextures
-  float4 *dNodes = nullptr, *dTris = nullptr, *dShade = nullptr, *dMats = nullptr, *dWide = nullptr;
+  float4 *dNodes = nullptr, *dTris = nullptr, *dShade = nullptr, *dMats = nullptr, *dWide = nullptr,
+         *dOrd = nullptr, *dOrdLeaf = nullptr;
   float4* dTexels = nullptr;
   uint4* dTexInfo = nullptr;
   float2* dUvs = nullptr;
@@ -104,6 +105,8 @@ struct gbpt_scene {
     dfree(dMats);
     dfree(dLight);
     dfree(dWide);
+    dfree(dOrd);
+    dfree(dOrdLeaf);
     dfree(dTexels);
     dfree(dTexInfo);
     dfree(dUvs);
@@ -204,6 +207,20 @@ gbpt_status upload_wide(gbpt_scene* s) {
   return GBPT_OK;
 }
 
+// the ordered walk's tree, where the scene's tree allows it
+gbpt_status upload_ordered(gbpt_scene* s, const std::vector<float4>& tris) {
+  OrderedTree t;
+  if (!ordered_tree(s->bvh, &tris[0].x, &t)) return GBPT_OK;
+  CK(dalloc(&s->dOrd, t.nodes.size() / 4));
+  CK(dalloc(&s->dOrdLeaf, t.leaves.size() / 4));
+  CK(cudaMemcpy(s->dOrd, t.nodes.data(), t.nodes.size() * 4, cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(s->dOrdLeaf, t.leaves.data(), t.leaves.size() * 4, cudaMemcpyHostToDevice));
+  s->dev.ord = s->dOrd;
+  s->dev.ordLeaf = s->dOrdLeaf;
+  s->dev.ordRange = t.range;
+  return GBPT_OK;
+}
+
 gbpt_status upload_scene(gbpt_scene* s) {
   gbpt_status ids = check_texture_ids(s->mats, s->textures.size());
   if (ids != GBPT_OK) return ids;
@@ -257,6 +274,8 @@ gbpt_status upload_scene(gbpt_scene* s) {
     gbpt_status w = upload_wide(s);
     if (w != GBPT_OK) return w;
   }
+  gbpt_status od = upload_ordered(s, tris);
+  if (od != GBPT_OK) return od;
   gbpt_status tx = upload_textures(s);
   if (tx != GBPT_OK) return tx;
   s->uploaded = true;
@@ -353,6 +372,9 @@ struct gbpt_renderer {
     dfree(rb.ctr);
     dfree(rb.carry[0]);
     dfree(rb.carry[1]);
+    dfree(rb.open);
+    dfree(rb.check);
+    dfree(rb.fix);
     dfree(rb.conn);
     rb.connDepth = 0;
     dfree(ab.err);
@@ -466,16 +488,25 @@ RenderBuffers band_buffers(const RenderBuffers& rb, uint32_t b, uint32_t k, size
   x.carry[0] = rb.carry[0] + c0 * kCarryF4;
   x.carry[1] = rb.carry[1] + c0 * kCarryF4;
   x.carryCap = (uint32_t)(c1 - c0);
+  x.open += 2 * p0 + c0;
+  x.checkCap = rb.checkCap / k;
+  x.check += (size_t)b * x.checkCap * 2 * kCheckF4;
+  x.fix += (size_t)b * x.checkCap * 2;
   return x;
 }
 
 }  // namespace
 
+// records for k_verify per list: about one walk in 5,000 needs one; a list that
+// is full costs the walk the reference's own
+static uint32_t check_cap(size_t np) { return (uint32_t)std::max<size_t>(np / 64, 256); }
+
 uint64_t gbpt::renderer_bytes(uint32_t W, uint32_t H, const gbpt_params& p) {
   const size_t np = (size_t)W * H;
   const uint32_t cacheCap = std::max(1u, p.light_paths * (1 + p.light_depth_max));
-  return np * (128 + 16 + 96 + 16 + 48 + 16 + 8) + np * (12 * 10 + 4 * 2 + 4 * 5) + (size_t)cacheCap * 192 +
-         std::max<size_t>(std::min<size_t>(np, walk_lanes()), 256) * (2 * kCarryF4 + 1) * 16 +
+  return np * (128 + 16 + 96 + 16 + 48 + 16 + 8 + 8) + np * (12 * 10 + 4 * 2 + 4 * 5) + (size_t)cacheCap * 192 +
+         std::max<size_t>(std::min<size_t>(np, walk_lanes()), 256) * (2 * kCarryF4 * 16 + 16 + 4) +
+         (size_t)check_cap(np) * 2 * (kCheckF4 * 16 + 4) +
          np * 16 * (std::max(std::max(p.eye_depth_max, p.pt_depth_max), 2u) - 1);
 }
 
@@ -515,6 +546,10 @@ gbpt_status ensure_alloc(gbpt_renderer* r) {
   CK(dalloc(&r->rb.cache[1], (size_t)cacheCap * 6));
   CK(dalloc(&r->rb.carry[0], (size_t)r->rb.carryCap * kCarryF4));
   CK(dalloc(&r->rb.carry[1], (size_t)r->rb.carryCap * kCarryF4));
+  CK(dalloc(&r->rb.open, 2 * cap + r->rb.carryCap));  // extension and connection rays, resumed walks
+  r->rb.checkCap = check_cap(cap);
+  CK(dalloc(&r->rb.check, (size_t)r->rb.checkCap * 2 * kCheckF4));
+  CK(dalloc(&r->rb.fix, (size_t)r->rb.checkCap * 2));
   CK(dalloc(&r->rb.ctr, kMaxBands));
   CK(cudaMemsetAsync(r->rb.ctr, 0, sizeof(DevCounters) * kMaxBands, r->st));
   r->rb.lctr = r->rb.ctr;
@@ -712,6 +747,10 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
     CK(cudaMemsetAsync(r->rb.hist, 0, (size_t)a.tilesX * ((r->H + 7) / 8) * 32, r->st));
   a.counting = r->counting ? 1u : 0u;
   const DevScene& S = s->dev;
+  // the ordered walk answers as the reference's but does not count its pops,
+  // and is exact for origins within the scene's range
+  a.ordered = S.ord && S.traversal == 0 && !a.counting && std::fabs(cam->pos[0]) <= S.ordRange &&
+              std::fabs(cam->pos[1]) <= S.ordRange && std::fabs(cam->pos[2]) <= S.ordRange;
   cudaStream_t st = r->st;
   // filter-only mode: frames past "Render Iteration" trace nothing and only
   // filter again (src/cudaRTBDPTStreamBilat.cu:1278)
@@ -807,8 +846,18 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
     const bool tailRun = K < D || carrying || a.tailBelow > 0.f;
     auto bounces = [&](const RenderBuffers& rbx, cudaStream_t sx, bool mk) -> gbpt_status {
       int in = 0;
+      // walks the frame takes as they ended are checked: the bounce launches'
+      // on a stream of their own from the last walk on (in a frame of one band)
+      const bool checks = checks_walks(S, a);
+      const bool aside = checks && mk && tailRun && K > 0;
       for (uint32_t d = 0; d < K; d++) {
         CK(launch_walk(S, a, rbx, in, d > 0 ? (int)((d - 1) & 1u) : -1, (int)(d & 1u), d, sx));
+        if (aside && d + 1 == K) {
+          CK(cudaEventRecord(r->evFork, sx));
+          CK(cudaStreamWaitEvent(r->stBand[0], r->evFork, 0));
+          CK(launch_verify(S, rbx, 0, r->stBand[0]));
+          CK(cudaEventRecord(r->evJoin[0], r->stBand[0]));
+        }
         if (mk) mark(r, kPhTrace, tm);
         CK(launch_shade(S, a, rbx, in, d, tailRun && d + 1 == K, sx));
         if (mk) mark(r, kPhShade, tm);
@@ -820,6 +869,14 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
         // shadow rays of the last bounce (none in practice: paths at the depth cap
         // terminate without connecting; kept so the sequence needs no special case)
         CK(launch_walk(S, a, rbx, -1, (int)((D - 1) & 1u), (int)(D & 1u), D, sx));
+      }
+      if (checks) {
+        if (aside)
+          CK(cudaStreamWaitEvent(sx, r->evJoin[0], 0));
+        else
+          CK(launch_verify(S, rbx, 0, sx));
+        CK(launch_verify(S, rbx, 1, sx));
+        CK(launch_tail_again(S, a, rbx, K, sx));
       }
       CK(launch_fold(rbx, sx));
       return GBPT_OK;

@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "../../include/gbpt.h"
+#include "ordered.h"
 
 namespace gbpt {
 
@@ -24,6 +25,11 @@ bool build_bvh(const gbpt_vertex* verts, const gbpt_triangle* tris, uint32_t nt,
 // per node (lo.x[4], lo.y[4], lo.z[4], hi.x[4], hi.y[4], hi.z[4], code[4] as
 // uint bits, 4 zeros); see DevScene in launch.h for the child codes.
 std::vector<float> collapse_wide(const HostBVH& bvh);
+
+// false: the scene keeps the reference's walk (empty children, boxes that are
+// not nested, more than 2^24 nodes, depth, extreme coordinates).  tris: 16
+// words per triangle in BVH order (p0, pad, p1 - p0, pad, p2 - p0, 5 pads).
+bool ordered_tree(const HostBVH& bvh, const float* tris, OrderedTree* out);
 
 // sqrt(mean((a - b)^2)) over n floats in device memory, summed in double on
 // `stream` (a cudaStream_t); image.cu

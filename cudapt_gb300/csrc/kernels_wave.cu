@@ -32,6 +32,7 @@
 #include <cstdlib>
 
 #include "launch.h"
+#include "ordered.cuh"
 #include "shade.cuh"
 #include "texture.cuh"
 #include "trace.cuh"
@@ -235,6 +236,7 @@ __device__ __forceinline__ LV load_lv(const float4* c) {
 // out exactly as the reference's stable remove_if does: a surviving path's
 // position in the stream equals the number of surviving paths with a lower
 // index, i.e. an exclusive scan of the "alive" flags.
+template <bool kOrdered>
 __global__ void __launch_bounds__(1024) k_light(DevScene S, FrameArgs a, float4* cache, uint32_t cacheCap,
                                                 DevCounters* ctr) {
   using namespace gb;
@@ -296,7 +298,12 @@ __global__ void __launch_bounds__(1024) k_light(DevScene S, FrameArgs a, float4*
         float4* cs = cache + 6 * (size_t)slot;
         TraceHit h;
         uint32_t nn = 0, nt = 0;
-        if (!trace_ref<false, false>(S, orig, dir, kInf, kBias, false, h, nn, nt)) {
+        bool hit;
+        if constexpr (kOrdered)
+          hit = trace_ord(S, orig, dir, kInf, kBias, h);
+        else
+          hit = trace_ref<false, false>(S, orig, dir, kInf, kBias, false, h, nn, nt);
+        if (!hit) {
           const float4* home = cache + 6 * (size_t)x;  // :358-362
           for (int k = 0; k < 6; k++) cs[k] = home[k];
           alive = false;
@@ -375,6 +382,7 @@ __global__ void k_camera(FrameArgs a, RenderBuffers b) {
     b.ctr->fetchT = 0;
     b.ctr->carryN[0] = b.ctr->carryN[1] = b.ctr->carryN[2] = 0;
     b.ctr->fetchTail = 0;
+    b.ctr->openN = b.ctr->checkN[0] = b.ctr->checkN[1] = b.ctr->fixN = 0;
     b.ctr->tailAt = 0xFFFFFFFFu;
   }
   if (i >= b.count) return;
@@ -457,9 +465,15 @@ __device__ __forceinline__ void warp_add_u64(unsigned long long* dst, uint32_t v
 // (refill 8): 190.0 / 172.3 / 147.4, 12: 195.1 / 177.8 / 150.9, 16: 196.5 /
 // 178.1 / 151.3, 24 (refill 4): 195.2 / 178.3 / 151.4; wide order 2: 170.0 /
 // 180.7 / 159.2, 4: 171.2 / 181.8 / 157.4
-template <bool kWide>
+template <int kKind>
 __host__ __device__ constexpr int walk_steps() {
-  return kWide ? 2 : 16;
+  return kKind == kWalkOrd ? 4 : kKind == kWalkWide ? 2 : 16;
+}
+// reference walk steps (pops) that one step stands for: an ordered step is a
+// wide node and a leaf, in place of 6 pops on average
+template <int kKind>
+__host__ __device__ constexpr uint32_t step_pops() {
+  return kKind == kWalkOrd ? 6u : 1u;
 }
 
 // Word 3.w of a carry record: the path's depth for an extension walk, this
@@ -467,29 +481,44 @@ __host__ __device__ constexpr int walk_steps() {
 // {origin, slot} {direction, maxDist} {contribution, bounce} instead of the path.
 constexpr uint32_t kShadowRec = 0xFFFFFFFFu;
 
+// Words of the list of walks k_resolve answers: the item of a launch's wave,
+// of its connection queue, or of the carry records it resumed.
+constexpr uint32_t kOpenShadow = 0x40000000u, kOpenCarried = 0x80000000u, kOpenItem = 0x3FFFFFFFu;
+
 // One carried walk to carry record r (out of line: it runs for a few walks
 // per launch, and keeping it out of the walk loop keeps that loop's
 // registers): three float4 of the walk's ray at src, src + stride, src +
 // 2 * stride (the path of a wave, or a connection record), the fourth at src
 // + 3 * stride (the path's carried emission and depth) or the connection tag,
-// then the walk's state and its node stack.
-__device__ __noinline__ void save_carry(float4* r, const float4* src, size_t stride, bool shadow, float minT,
-                                        uint32_t best, float bu, float bv, float bw, uint32_t steps, uint32_t tos,
-                                        int sp, const uint32_t* stack) {
+// then the walk's state (two float4) and its node stack (n words).
+__device__ __noinline__ void save_carry(float4* r, const float4* src, size_t stride, bool shadow, float4 state0,
+                                        float4 state1, const uint32_t* stack, uint32_t n) {
   r[0] = src[0];
   r[1] = src[stride];
   r[2] = src[2 * stride];
   r[3] = shadow ? make_float4(0.f, 0.f, 0.f, __uint_as_float(kShadowRec)) : src[3 * stride];
-  r[4] = make_float4(minT, __uint_as_float(best), bu, bv);
-  r[5] = make_float4(bw, __uint_as_float(steps), __uint_as_float(tos), __int_as_float(sp));
-  for (int k = 0; k < 8; k++)
+  r[4] = state0;
+  r[5] = state1;
+  for (uint32_t k = 0; 4 * k < n; k++)
     r[6 + k] = make_float4(__uint_as_float(stack[4 * k]), __uint_as_float(stack[4 * k + 1]),
                            __uint_as_float(stack[4 * k + 2]), __uint_as_float(stack[4 * k + 3]));
 }
+__device__ __forceinline__ void save_walk(float4* r, const float4* src, size_t stride, bool shadow, const Walk& w,
+                                          const uint32_t* stack) {
+  save_carry(r, src, stride, shadow, make_float4(w.minT, __uint_as_float(w.best), w.bu, w.bv),
+             make_float4(w.bw, __uint_as_float(w.steps), __uint_as_float(w.tos), __int_as_float(w.sp)), stack, 32);
+}
+__device__ __forceinline__ void save_walk(float4* r, const float4* src, size_t stride, bool shadow, const OrdWalk& w,
+                                          const uint2* stack) {
+  save_carry(r, src, stride, shadow, make_float4(w.minT, __uint_as_float(w.best), w.bu, w.bv),
+             make_float4(__uint_as_float(w.gA), __uint_as_float(w.gB), __uint_as_float(w.bound), __int_as_float(w.sp)),
+             reinterpret_cast<const uint32_t*>(stack), 2u * (uint32_t)w.sp);
+}
+static_assert(kCarryF4 >= 6 + 8 && kCarryF4 >= 6 + kOrdStack / 2, "carry record holds either walk");
 
 // The walk of carry record r, resumed at the step where it stopped; true for
 // a connection walk (any hit up to its maxDist).
-__device__ __forceinline__ bool resume_walk(const float4* r, Walk& w, uint32_t* stack) {
+__device__ __forceinline__ bool resume_walk(const DevScene& S, const float4* r, Walk& w, uint32_t* stack) {
   const float4 r1 = r[1];
   const bool shadow = __float_as_uint(r[3].w) == kShadowRec;
   w.init(ld3(r[0]), ld3(r1), shadow ? r1.w : gb::kInf, gb::kBias, stack);
@@ -512,6 +541,28 @@ __device__ __forceinline__ bool resume_walk(const float4* r, Walk& w, uint32_t* 
   }
   return shadow;
 }
+__device__ __forceinline__ bool resume_walk(const DevScene& S, const float4* r, OrdWalk& w, uint2* stack) {
+  const float4 r1 = r[1];
+  const bool shadow = __float_as_uint(r[3].w) == kShadowRec;
+  start_walk<kWalkOrd>(S, w, ld3(r[0]), ld3(r1), 0.f, shadow, stack);
+  const float4 q = r[4], z = r[5];
+  w.minT = q.x;
+  w.best = __float_as_uint(q.y);
+  w.bu = q.z;
+  w.bv = q.w;
+  w.gA = __float_as_uint(z.x);
+  w.gB = __float_as_uint(z.y);
+  w.bound = __float_as_uint(z.z);
+  w.sp = __float_as_int(z.w);
+  w.rescale(S);
+#pragma unroll 1
+  for (int k = 0; 2 * k < w.sp; k++) {
+    const float4 e = r[6 + k];
+    stack[2 * k] = make_uint2(__float_as_uint(e.x), __float_as_uint(e.y));
+    stack[2 * k + 1] = make_uint2(__float_as_uint(e.z), __float_as_uint(e.w));
+  }
+  return shadow;
+}
 
 // An unoccluded connection: its contribution into the slot's entry for the
 // bounce that made it (summed with the path's other connections, in bounce
@@ -526,6 +577,31 @@ __device__ __forceinline__ void connection_reached(const RenderBuffers& b, uint3
 // counter of launch L + 1 is reset by launch L, after its last reader)
 __device__ __forceinline__ uint32_t carried_of(const RenderBuffers& b, uint32_t launch) {
   return b.carry[0] ? min(b.ctr->carryN[launch % 3u], b.carryCap) : 0u;
+}
+
+// What becomes of an ordered walk that ended past the reference's pop bound
+// (about 0.01-0.02 % of them; hardly any really run out of pops): the
+// reference's walk at once (scenes too small to run out, where only origins
+// outside the walk's range come here); a list that k_resolve answers before
+// the launch is shaded (the modes whose shading adds to per-path state); or
+// taken as it is, with a record of the path at this point that k_verify checks
+// while the frame goes on (every other mode).
+enum : uint32_t { kOpenNow = 0, kOpenList = 1, kOpenCheck = 2 };
+
+// A record to check: {path's four float4, or the connection's three and its
+// tag} {t, triangle, u, v; t -1: no hit}.  list 0: bounce launches, 1: the tail
+// kernel.  False when the list is full.
+__device__ __forceinline__ bool note_check(const RenderBuffers& b, uint32_t list, float4 r0, float4 r1, float4 r2,
+                                           float4 r3, float4 answer) {
+  const uint32_t k = atomicAdd(&b.ctr->checkN[list], 1u);
+  if (k >= b.checkCap) return false;
+  float4* r = b.check + ((size_t)list * b.checkCap + k) * kCheckF4;
+  r[0] = r0;
+  r[1] = r1;
+  r[2] = r2;
+  r[3] = r3;
+  r[4] = answer;
+  return true;
 }
 
 // Carrying (reference order only): once the launch's ray queue is empty, a
@@ -543,12 +619,12 @@ __device__ __forceinline__ uint32_t carried_of(const RenderBuffers& b, uint32_t 
 // connections may now finish out of order).  The filter-only mode's bounce-0
 // connections, whose direct-light sample is read by the next bounce's
 // shading, are never carried.
-template <bool kCount, bool kWide>
+template <bool kCount, int kKind>
 __global__ void __launch_bounds__(kBlock, 4) k_walk(DevScene S, RenderBuffers b, int in, int shIn,
                                                               int shReset, uint32_t bilat, uint32_t kRefill,
-                                                              uint32_t launch, uint32_t carrySteps) {
+                                                              uint32_t launch, uint32_t carrySteps, uint32_t later) {
   if (b.ctr->tailAt <= launch) return;  // the frame's tail kernel carries this bounce
-  const uint32_t nC = (!kWide && in >= 0 && launch > 0) ? carried_of(b, launch - 1) : 0u;
+  const uint32_t nC = (kKind != kWalkWide && in >= 0 && launch > 0) ? carried_of(b, launch - 1) : 0u;
   const uint32_t nE = (in >= 0) ? b.ctr->wave[in] : 0u;
   const uint32_t nS = (shIn >= 0) ? b.ctr->shadow[shIn] : 0u;
   const uint32_t nCE = nC + nE;
@@ -565,20 +641,21 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(DevScene S, RenderBuffers b,
   const float4* __restrict__ sh = b.sh[shIn >= 0 ? shIn : 0];
   const float4* prev = b.carry[(launch + 1) & 1u];  // launch - 1's carried walks
   const uint32_t lane = threadIdx.x & 31;
-  typename WalkOf<kWide>::type w;
-  typename WalkOf<kWide>::Entry stack[WalkOf<kWide>::kDepth];
+  typename WalkOf<kKind>::type w;
+  typename WalkOf<kKind>::Entry stack[WalkOf<kKind>::kDepth];
   bool has = false, drained = false, any = false, res = false;
   uint32_t item = 0, nnE = 0, ntE = 0, nnS = 0, ntS = 0;
   uint32_t dryFor = 0;  // walk steps since this warp found the queue empty
   for (;;) {
     const uint32_t idle = __ballot_sync(0xffffffffu, !has);
     if (idle == 0xffffffffu && drained) break;
-    if constexpr (!kWide) {
+    if constexpr (kKind == kWalkOrd) w.stop_long();
+    if constexpr (kKind != kWalkWide) {
       if (carrySteps && drained && in >= 0) {
         // once per warp, carrySteps steps after it found the queue empty: its
         // walks still running take carry records with one atomic for the warp
         // (walks that find the buffer full finish here)
-        if (dryFor >= carrySteps && dryFor < carrySteps + walk_steps<kWide>()) {
+        if (dryFor >= carrySteps && dryFor < carrySteps + walk_steps<kKind>() * step_pops<kKind>()) {
           const float4* src = res ? prev + (size_t)item * kCarryF4 : (any ? sh + 3 * (size_t)item : wv.o + item);
           const bool want = has && !(any && bilat && __float_as_uint(src[2].w) == 0u);
           const uint32_t m = __ballot_sync(0xffffffffu, want);
@@ -586,13 +663,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(DevScene S, RenderBuffers b,
           if (m && lane == 0) c0 = atomicAdd(&b.ctr->carryN[launch % 3u], (uint32_t)__popc(m));
           c0 = __shfl_sync(0xffffffffu, c0, 0) + __popc(m & lanemask_lt());
           if (want && c0 < b.carryCap) {
-            save_carry(b.carry[launch & 1u] + (size_t)c0 * kCarryF4, src, (res || any) ? 1 : (size_t)(wv.d - wv.o),
-                       any && !res, w.minT, w.best, w.bu, w.bv, w.bw, w.steps, w.tos, w.sp, stack);
+            save_walk(b.carry[launch & 1u] + (size_t)c0 * kCarryF4, src, (res || any) ? 1 : (size_t)(wv.d - wv.o),
+                      any && !res, w, stack);
             if (res || !any) b.hit[res ? nE + item : item] = make_float4(-2.f, 0.f, 0.f, 0.f);
             has = false;
           }
         }
-        dryFor += walk_steps<kWide>();
+        dryFor += walk_steps<kKind>() * step_pops<kKind>();
       }
     }
     if (!drained && (idle == 0xffffffffu || __popc(idle) >= kRefill)) {
@@ -609,12 +686,12 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(DevScene S, RenderBuffers b,
           res = !any && k < nS + nC;
           item = any ? k : (res ? k - nS : k - nS - nC);
           if (res) {
-            if constexpr (!kWide) any = resume_walk(prev + (size_t)item * kCarryF4, w, stack);
+            if constexpr (kKind != kWalkWide) any = resume_walk(S, prev + (size_t)item * kCarryF4, w, stack);
           } else if (any) {
             const float4 A = sh[3 * (size_t)item], B = sh[3 * (size_t)item + 1];
-            w.init(ld3(A), ld3(B), B.w, gb::kBias, stack);
+            start_walk<kKind>(S, w, ld3(A), ld3(B), B.w, true, stack);
           } else {
-            w.init(ld3(wv.o[item]), ld3(wv.d[item]), gb::kInf, gb::kBias, stack);
+            start_walk<kKind>(S, w, ld3(wv.o[item]), ld3(wv.d[item]), gb::kInf, false, stack);
           }
         }
       }
@@ -622,20 +699,46 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(DevScene S, RenderBuffers b,
     // walk_steps() steps per refill check: the ballot and refill test are paid
     // once for them (a lane whose walk ends in the first waits out the rest)
 #pragma unroll 1
-    for (int u = 0; u < walk_steps<kWide>(); u++) {
+    for (int u = 0; u < walk_steps<kKind>(); u++) {
       // one inlined walk step for both ray kinds (a runtime any-hit flag), so a
       // warp holding extension and shadow rays does not run two copies of it;
       // the counting variant keeps separate counters per kind
       bool fin = false;
-      if (has) {
+      if constexpr (kKind == kWalkOrd) {
+        fin = w.step_warp(S, stack, has);
+      } else if (has) {
         if (kCount)
-          fin = any ? w.template step<kCount>(S, stack, true, nnS, ntS) : w.template step<kCount>(S, stack, false, nnE, ntE);
+          fin = any ? step_walk<kKind, kCount>(S, w, stack, true, nnS, ntS)
+                    : step_walk<kKind, kCount>(S, w, stack, false, nnE, ntE);
         else
-          fin = w.template step<kCount>(S, stack, any, nnE, ntE);
+          fin = step_walk<kKind, kCount>(S, w, stack, any, nnE, ntE);
       }
       if (fin) {
         has = false;
-        if (any) {
+        bool open = false;
+        if constexpr (kKind == kWalkOrd) {
+          if (w.capped()) {
+            open = later == kOpenList;
+            bool now = later == kOpenNow || w.bound >= kPopStop;  // an unfinished walk has no answer to take
+            if (later == kOpenCheck && !now) {
+              const float4* q = res ? prev + (size_t)item * kCarryF4 : any ? sh + 3 * (size_t)item : wv.o + item;
+              const size_t st = (res || any) ? 1 : (size_t)(wv.d - wv.o);
+              now = !note_check(b, 0, q[0], q[st], q[2 * st],
+                                any ? make_float4(0.f, 0.f, 0.f, __uint_as_float(kShadowRec)) : q[3 * st],
+                                make_float4(w.hit() ? w.minT : -1.f, __uint_as_float(w.best), w.bu, w.bv));
+            }
+            if (!open && now) {
+              TraceHit h;
+              uint32_t nn = 0, nt = 0;
+              const float far = any ? (res ? prev + (size_t)item * kCarryF4 : sh + 3 * (size_t)item)[1].w : gb::kInf;
+              const bool hit = trace_ref<false, false>(S, w.o, w.d, far, gb::kBias, false, h, nn, nt);
+              w.settle(hit, make_float4(h.t, __uint_as_float(h.tri), h.u, h.v));
+            }
+          }
+        }
+        if (open) {
+          b.open[atomicAdd(&b.ctr->openN, 1u)] = item | (res ? kOpenCarried : any ? kOpenShadow : 0u);
+        } else if (any) {
           const float4* q = res ? prev + (size_t)item * kCarryF4 : sh + 3 * (size_t)item;
           if (!w.hit()) connection_reached(b, bilat, q[0], q[2]);  // unoccluded: it counts (:716-721)
           if (res) b.hit[nE + item] = make_float4(-2.f, 0.f, 0.f, 0.f);
@@ -786,6 +889,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_shade(DevScene S, FrameArgs a, Re
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     atomicAdd(&b.ctr->rays, (unsigned long long)n);  // resumed walks were counted by their own launch
     b.ctr->fetchT = 0;  // for the next walk (next bounce's rays + this bounce's shadow rays)
+    b.ctr->openN = 0;
     if (attach == 2u) b.ctr->tailAt = launch + 1;
   }
   const Wave w = b.wave[in];
@@ -873,17 +977,21 @@ enum : uint32_t { kIdle = 0, kPathExt = 1, kPathShadow = 2 };
 // 192.7.  Three CTAs per SM (80 registers, some spill) against two (116
 // registers): interior 167.0 -> 170.0, Cornell 195.6 -> 193.6 Mpaths/s; four
 // (64 registers): hall 195.9 -> 194.6, Cornell 190.4 -> 183.1.
-__host__ __device__ constexpr int tail_steps() { return 64; }
+template <int kKind>
+__host__ __device__ constexpr int tail_steps() {
+  return kKind == kWalkOrd ? 16 : 64;
+}
 
-template <bool kCount, bool kWide>
+template <bool kCount, int kKind>
 __global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, RenderBuffers b, uint32_t K,
-                                                   uint32_t kRefill) {
+                                                   uint32_t kRefill, uint32_t later, uint32_t again) {
   // t: the launch the bounce launches stopped before (the device switch or K)
   const uint32_t t = min(b.ctr->tailAt, K);
   const int in = (int)(t & 1u);
   const int shIn = t > 0 ? (int)((t - 1) & 1u) : -1;
-  const uint32_t n = b.ctr->wave[in];
-  const uint32_t nCarry = t > 0 ? carried_of(b, t - 1) : 0u;
+  // again: only the paths whose recorded answer k_verify corrected, from there on
+  const uint32_t n = again ? 0u : b.ctr->wave[in];
+  const uint32_t nCarry = again ? b.ctr->fixN : t > 0 ? carried_of(b, t - 1) : 0u;
   const float4* carried = b.carry[(t + 1) & 1u];  // launch t - 1's
   const uint32_t total = n + nCarry;
   const uint32_t cacheSize = b.lctr->cacheSize[a.cacheSel];
@@ -891,8 +999,8 @@ __global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, Ren
   const float4* __restrict__ sh = b.sh[shIn >= 0 ? shIn : 0];
   const Wave wv = b.wave[in];
   const uint32_t lane = threadIdx.x & 31;
-  typename WalkOf<kWide>::type w;
-  typename WalkOf<kWide>::Entry stack[WalkOf<kWide>::kDepth];
+  typename WalkOf<kKind>::type w;
+  typename WalkOf<kKind>::Entry stack[WalkOf<kKind>::kDepth];
   PathIO io;
   uint32_t mode = kIdle;
   bool drained = false, resumed = false;
@@ -900,6 +1008,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, Ren
   for (;;) {
     const uint32_t idle = __ballot_sync(0xffffffffu, mode == kIdle);
     if (idle == 0xffffffffu && drained) break;
+    if constexpr (kKind == kWalkOrd) w.stop_long();
     if (!drained && (idle == 0xffffffffu || __popc(idle) >= kRefill)) {
       const uint32_t cnt = __popc(idle);
       uint32_t base = 0;
@@ -911,8 +1020,33 @@ __global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, Ren
         if (j >= n && j < total) {  // a carried walk: resume it where it stopped
           const float4* r = carried + (size_t)(j - n) * kCarryF4;
           resumed = true;
-          if constexpr (!kWide) {
-            if (resume_walk(r, w, stack)) {  // a connection alone, without its path
+          if (kKind == kWalkOrd && again) {
+            const uint32_t k = j - n;
+            r = b.check + (size_t)b.fix[k] * kCheckF4;
+            io.o = r[0];
+            io.d = r[1];
+            io.t = r[2];
+            io.s = r[3];
+            mode = kPathExt;
+            // a path corrected at an earlier bounce as well starts there
+            for (uint32_t m = 0; m < nCarry; m++) {
+              const float4* q = b.check + (size_t)b.fix[m] * kCheckF4;
+              if (__float_as_uint(q[0].w) == __float_as_uint(io.o.w) &&
+                  __float_as_uint(q[3].w) < __float_as_uint(io.s.w))
+                mode = kIdle;
+            }
+            if constexpr (kKind == kWalkOrd) {
+              start_walk<kKind>(S, w, ld3(io.o), ld3(io.d), gb::kInf, false, stack);
+              w.gB = 0u;  // over, with the corrected answer
+              w.settle(r[4].x >= 0.f, r[4]);
+            }
+            resumed = mode != kIdle;
+            if (a.gbuffer && resumed && __float_as_uint(io.s.w) == 0u) {  // as k_camera leaves them
+              float4* g = b.gbuf + 3 * (size_t)__float_as_uint(io.o.w);
+              g[0] = g[1] = g[2] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+          } else if constexpr (kKind != kWalkWide) {
+            if (resume_walk(S, r, w, stack)) {  // a connection alone, without its path
               io.shA = r[0];
               io.shB = r[1];
               io.shC = r[2];
@@ -936,22 +1070,44 @@ __global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, Ren
             io.shB = sh[3 * (size_t)j + 1];
             io.shC = sh[3 * (size_t)j + 2];
             mode = kPathShadow;
-            w.init(ld3(io.shA), ld3(io.shB), io.shB.w, gb::kBias, stack);
+            start_walk<kKind>(S, w, ld3(io.shA), ld3(io.shB), io.shB.w, true, stack);
           } else {
             mode = kPathExt;
-            w.init(ld3(io.o), ld3(io.d), gb::kInf, gb::kBias, stack);
+            start_walk<kKind>(S, w, ld3(io.o), ld3(io.d), gb::kInf, false, stack);
           }
         }
       }
     }
-    if (mode == kIdle) continue;
+    if (kKind != kWalkOrd && mode == kIdle) continue;
     const bool anyHit = mode == kPathShadow;
     bool done = false;
+    if constexpr (kKind == kWalkOrd) {
+      // the warp's walks advance together until they are all over, at most tail_steps times
 #pragma unroll 1
-    for (int u = 0; u < tail_steps() && !done; u++)
-      done = kCount ? (anyHit ? w.template step<kCount>(S, stack, true, nnS, ntS)
-                              : w.template step<kCount>(S, stack, false, nnE, ntE))
-                    : w.template step<kCount>(S, stack, anyHit, nnE, ntE);
+      for (int u = 0; u < tail_steps<kKind>(); u++) {
+        done = w.step_warp(S, stack, mode != kIdle);
+        if (__all_sync(0xffffffffu, done || mode == kIdle)) break;
+      }
+      if (mode == kIdle) continue;
+      if (done && w.capped()) {
+        const float4 got = make_float4(w.hit() ? w.minT : -1.f, __uint_as_float(w.best), w.bu, w.bv);
+        const bool noted =
+            later == kOpenCheck && w.bound < kPopStop &&
+            (anyHit ? note_check(b, 1, io.shA, io.shB, io.shC, make_float4(0.f, 0.f, 0.f, __uint_as_float(kShadowRec)), got)
+                    : note_check(b, 1, io.o, io.d, io.t, io.s, got));
+        if (!noted) {
+          TraceHit h;
+          uint32_t nn = 0, nt = 0;
+          const bool hit = trace_ref<false, false>(S, w.o, w.d, anyHit ? io.shB.w : gb::kInf, gb::kBias, false, h, nn, nt);
+          w.settle(hit, make_float4(h.t, __uint_as_float(h.tri), h.u, h.v));
+        }
+      }
+    } else
+#pragma unroll 1
+    for (int u = 0; u < tail_steps<kKind>() && !done; u++)
+      done = kCount ? (anyHit ? step_walk<kKind, kCount>(S, w, stack, true, nnS, ntS)
+                              : step_walk<kKind, kCount>(S, w, stack, false, nnE, ntE))
+                    : step_walk<kKind, kCount>(S, w, stack, anyHit, nnE, ntE);
     if (!done) continue;
     if (anyHit) {
       if (!w.hit()) connection_reached(b, a.bilat, io.shA, io.shC);  // unoccluded connection (:716-721)
@@ -962,7 +1118,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, Ren
       }
       shRays++;
       mode = kPathExt;  // the path's next extension ray
-      w.init(ld3(io.o), ld3(io.d), gb::kInf, gb::kBias, stack);
+      start_walk<kKind>(S, w, ld3(io.o), ld3(io.d), gb::kInf, false, stack);
       continue;
     }
     // closest hit of the path's current ray: shade it (a resumed walk was
@@ -977,9 +1133,9 @@ __global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, Ren
     } else {
       if (io.conn) {
         mode = kPathShadow;
-        w.init(ld3(io.shA), ld3(io.shB), io.shB.w, gb::kBias, stack);
+        start_walk<kKind>(S, w, ld3(io.shA), ld3(io.shB), io.shB.w, true, stack);
       } else {
-        w.init(ld3(io.o), ld3(io.d), gb::kInf, gb::kBias, stack);
+        start_walk<kKind>(S, w, ld3(io.o), ld3(io.d), gb::kInf, false, stack);
       }
     }
   }
@@ -990,6 +1146,101 @@ __global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, Ren
     warp_add_u64(&b.ctr->tris, ntE);
     warp_add_u64(&b.ctr->nodesS, nnS);
     warp_add_u64(&b.ctr->trisS, ntS);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Answers of the walks bounce launch `launch` listed, one block each, before it
+// is shaded.  On the 332,180-triangle hall about 150 of a launch's million
+// walks; 65 us, most of it the cold binary tree's latency level by level.
+__global__ void __launch_bounds__(kCapThreads) k_resolve(DevScene S, RenderBuffers b, int in, int shIn, uint32_t bilat,
+                                                         uint32_t launch) {
+  extern __shared__ float4 capMem[];
+  CapShared& c = *reinterpret_cast<CapShared*>(capMem);
+  if (b.ctr->tailAt <= launch) return;
+  const uint32_t n = b.ctr->openN, nE = (in >= 0) ? b.ctr->wave[in] : 0u;
+  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+    const uint32_t code = b.open[i], item = code & kOpenItem;
+    const bool res = (code & kOpenCarried) != 0u;
+    const float4* r = res ? b.carry[(launch + 1) & 1u] + (size_t)item * kCarryF4
+                          : (code & kOpenShadow) ? b.sh[shIn] + 3 * (size_t)item : nullptr;
+    const bool any = r && (!res || __float_as_uint(r[3].w) == kShadowRec);
+    const float4 A = r ? r[0] : b.wave[in].o[item], B = r ? r[1] : b.wave[in].d[item];
+    resolve_capped(S, c, ld3(A), ld3(B), any ? B.w : gb::kInf, gb::kBias, any);
+    if (threadIdx.x == 0) {
+      if (any) {
+        if (!c.found) connection_reached(b, bilat, A, r[2]);
+        if (res) b.hit[nE + item] = make_float4(-2.f, 0.f, 0.f, 0.f);
+      } else {
+        b.hit[res ? nE + item : item] = c.found ? c.answer : make_float4(-1.f, 0.f, 0.f, 0.f);
+      }
+    }
+  }
+}
+
+// Checks the recorded answers of one list, one block each.  A connection's
+// entry is set right here; a path whose closest hit was another gets its
+// record's answer corrected and joins the list the tail kernel runs again from
+// that bounce, which rewrites everything the path wrote from there on (its
+// connection entries, its end, its first-hit planes).  The bounce launches'
+// list is checked beside the tail kernel.
+__global__ void __launch_bounds__(kCapThreads) k_verify(DevScene S, RenderBuffers b, uint32_t list) {
+  extern __shared__ float4 capMem[];
+  CapShared& c = *reinterpret_cast<CapShared*>(capMem);
+  const uint32_t n = min(b.ctr->checkN[list], b.checkCap);
+  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+    const uint32_t rec = list * b.checkCap + i;
+    float4* r = b.check + (size_t)rec * kCheckF4;
+    const bool any = __float_as_uint(r[3].w) == kShadowRec;
+    const float4 A = r[0], B = r[1], got = r[4];
+    resolve_capped(S, c, ld3(A), ld3(B), any ? B.w : gb::kInf, gb::kBias, any);
+    if (threadIdx.x != 0) continue;
+    const bool hit = c.found != 0u, was = got.x >= 0.f;
+    if (any) {
+      if (hit != was) {
+        const float4 C = r[2];
+        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+        b.conn[(size_t)__float_as_uint(C.w) * b.cap + __float_as_uint(A.w)] = hit ? none : make_float4(C.x, C.y, C.z, 1.f);
+      }
+    } else if (hit != was || (hit && (c.answer.x != got.x || __float_as_uint(c.answer.y) != __float_as_uint(got.y)))) {
+      r[4] = hit ? c.answer : make_float4(-1.f, 0.f, 0.f, 0.f);
+      b.fix[atomicAdd(&b.ctr->fixN, 1u)] = rec;
+    }
+  }
+  if (list == 1u && blockIdx.x == 0 && threadIdx.x == 0) b.ctr->fetchTail = 0;  // for the tail kernel's second run
+}
+
+// ... and of caller-supplied rays (k_trace_rays marks them with triangle -2):
+// a block looks through 256 rays and answers the marked ones.
+__global__ void __launch_bounds__(kCapThreads) k_resolve_rays(DevScene S, const float* rays, uint32_t n, float maxDist,
+                                                              float eps, float* t, int32_t* tri, float* w, float* u,
+                                                              float* v) {
+  extern __shared__ float4 capMem[];
+  CapShared& c = *reinterpret_cast<CapShared*>(capMem);
+  __shared__ uint32_t list[kCapThreads], count;
+  for (uint32_t base = blockIdx.x * kCapThreads; base < n; base += gridDim.x * kCapThreads) {
+    const uint32_t i = base + threadIdx.x;
+    const bool open = i < n && tri[i] == -2;
+    if (!__syncthreads_or(open)) continue;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    if (open) list[atomicAdd(&count, 1u)] = i;
+    __syncthreads();
+    const uint32_t m = count;
+    for (uint32_t k = 0; k < m; k++) {
+      const uint32_t j = list[k];
+      const float* r = rays + 6 * (size_t)j;
+      resolve_capped(S, c, mk(r[0], r[1], r[2]), mk(r[3], r[4], r[5]), maxDist, eps, false);
+      if (threadIdx.x == 0) {
+        const float4 h = c.answer;
+        t[j] = c.found ? h.x : -1.f;
+        tri[j] = c.found ? (int32_t)__float_as_uint(h.y) : -1;
+        w[j] = c.found ? 1.f - h.z - h.w : 0.f;
+        u[j] = c.found ? h.z : 0.f;
+        v[j] = c.found ? h.w : 0.f;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -1154,6 +1405,13 @@ __global__ void k_trace_rays(DevScene S, const float* rays, uint32_t n, float ma
     h.w = wk.bw;
     h.u = wk.bu;
     h.v = wk.bv;
+  } else if (!kCount && S.ord && S.traversal == 0 && !cullback) {
+    bool open = false;
+    hit = trace_ord(S, mk(r[0], r[1], r[2]), mk(r[3], r[4], r[5]), maxDist, eps, h, &open);
+    if (open) {
+      tri[i] = -2;  // for k_resolve_rays
+      return;
+    }
   } else {
     hit = trace_ref<false, kCount>(S, mk(r[0], r[1], r[2]), mk(r[3], r[4], r[5]), maxDist, eps, cullback != 0, h,
                                    nn, nt);
@@ -1212,7 +1470,10 @@ int sm_count() {
 cudaError_t launch_light_pass(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, cudaStream_t st) {
   uint32_t threads = ((a.lightPaths + 31) / 32) * 32;
   if (threads == 0) threads = 32;
-  k_light<<<1, threads, 0, st>>>(S, a, b.cache[a.cacheSel], b.cacheCap, b.ctr);
+  if (a.ordered)
+    k_light<true><<<1, threads, 0, st>>>(S, a, b.cache[a.cacheSel], b.cacheCap, b.ctr);
+  else
+    k_light<false><<<1, threads, 0, st>>>(S, a, b.cache[a.cacheSel], b.cacheCap, b.ctr);
   note_launches(1);
   return cudaGetLastError();
 }
@@ -1224,15 +1485,15 @@ cudaError_t launch_camera(const FrameArgs& a, const RenderBuffers& b, cudaStream
 }
 
 // launch shapes, queried once per kernel
-template <bool kCount, bool kWide>
+template <bool kCount, int kKind>
 uint32_t walk_grid() {
-  static uint32_t g = grid_for((const void*)k_walk<kCount, kWide>);
+  static uint32_t g = grid_for((const void*)k_walk<kCount, kKind>);
   return g;
 }
 
-template <bool kCount, bool kWide>
+template <bool kCount, int kKind>
 uint32_t tail_grid() {
-  static uint32_t g = grid_for((const void*)k_tail<kCount, kWide>);
+  static uint32_t g = grid_for((const void*)k_tail<kCount, kKind>);
   return g;
 }
 
@@ -1248,17 +1509,35 @@ uint32_t persistent_grid(uint32_t full, uint32_t ctasPerSm) {
   return std::min(full, (uint32_t)sm_count() * ctasPerSm);
 }
 
-template <bool kCount, bool kWide>
+template <bool kCount, int kKind>
 void walk_variant(const DevScene& S, const RenderBuffers& b, int in, int shIn, int shReset, uint32_t bilat,
-                  uint32_t refill, uint32_t ctas, uint32_t launch, uint32_t carrySteps, cudaStream_t st) {
-  const uint32_t g = persistent_grid(walk_grid<kCount, kWide>(), ctas);
-  k_walk<kCount, kWide><<<g, kBlock, 0, st>>>(S, b, in, shIn, shReset, bilat, refill, launch, carrySteps);
+                  uint32_t refill, uint32_t ctas, uint32_t launch, uint32_t carrySteps, uint32_t later,
+                  cudaStream_t st) {
+  const uint32_t g = persistent_grid(walk_grid<kCount, kKind>(), ctas);
+  k_walk<kCount, kKind><<<g, kBlock, 0, st>>>(S, b, in, shIn, shReset, bilat, refill, launch, carrySteps, later);
 }
 
-template <bool kCount, bool kWide>
-void tail_variant(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K, cudaStream_t st) {
-  const uint32_t g = persistent_grid(tail_grid<kCount, kWide>(), a.walkCtas);
-  k_tail<kCount, kWide><<<g, kBlock, 0, st>>>(S, a, b, K, walk_refill_for(a.refill, kWide));
+template <bool kCount, int kKind>
+void tail_variant(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K, uint32_t later,
+                  uint32_t again, cudaStream_t st) {
+  const uint32_t g = persistent_grid(tail_grid<kCount, kKind>(), a.walkCtas);
+  k_tail<kCount, kKind><<<g, kBlock, 0, st>>>(S, a, b, K, walk_refill_for(a.refill, kKind == kWalkWide), later, again);
+}
+
+// one block per SM (its lists take half of an SM's shared memory): opens the
+// kernel for that much once per device context
+template <typename Kern>
+cudaError_t cap_launchable(Kern kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CapShared));
+}
+
+// what becomes of walks past the pop bound: a tree of up to 2048 nodes cannot
+// have any; the filter-only mode's direct-light sample and the learned
+// allocator's path-length counts are added to as a path is shaded, so their
+// paths cannot be run again
+uint32_t open_rule(const DevScene& S, const FrameArgs& a) {
+  if (S.nodeN <= kPopCap) return kOpenNow;
+  return a.bilat || a.moments ? kOpenList : kOpenCheck;
 }
 
 cudaError_t launch_walk(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, int in, int shIn,
@@ -1267,12 +1546,20 @@ cudaError_t launch_walk(const DevScene& S, const FrameArgs& a, const RenderBuffe
   const bool wide = S.traversal == 1 && S.wide;
   const uint32_t rf = walk_refill_for(a.refill, wide);
   const uint32_t cs = b.carry[0] ? a.carrySteps : 0u;
-  if (a.counting) {
-    if (wide) walk_variant<true, true>(S, b, in, shIn, shReset, sd, rf, a.walkCtas, launch, 0u, st);
-    else walk_variant<true, false>(S, b, in, shIn, shReset, sd, rf, a.walkCtas, launch, cs, st);
+  if (a.ordered) {
+    walk_variant<false, kWalkOrd>(S, b, in, shIn, shReset, sd, rf, a.walkCtas, launch, cs, open_rule(S, a), st);
+    if (open_rule(S, a) == kOpenList) {
+      const cudaError_t e = cap_launchable(k_resolve);
+      if (e != cudaSuccess) return e;
+      k_resolve<<<sm_count(), kCapThreads, sizeof(CapShared), st>>>(S, b, in, shIn, sd, launch);
+      note_launches(1);
+    }
+  } else if (a.counting) {
+    if (wide) walk_variant<true, kWalkWide>(S, b, in, shIn, shReset, sd, rf, a.walkCtas, launch, 0u, 0u, st);
+    else walk_variant<true, kWalkRef>(S, b, in, shIn, shReset, sd, rf, a.walkCtas, launch, cs, 0u, st);
   } else {
-    if (wide) walk_variant<false, true>(S, b, in, shIn, shReset, sd, rf, a.walkCtas, launch, 0u, st);
-    else walk_variant<false, false>(S, b, in, shIn, shReset, sd, rf, a.walkCtas, launch, cs, st);
+    if (wide) walk_variant<false, kWalkWide>(S, b, in, shIn, shReset, sd, rf, a.walkCtas, launch, 0u, 0u, st);
+    else walk_variant<false, kWalkRef>(S, b, in, shIn, shReset, sd, rf, a.walkCtas, launch, cs, 0u, st);
   }
   note_launches(1);
   return cudaGetLastError();
@@ -1280,28 +1567,51 @@ cudaError_t launch_walk(const DevScene& S, const FrameArgs& a, const RenderBuffe
 
 cudaError_t launch_tail(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K, cudaStream_t st) {
   const bool wide = S.traversal == 1 && S.wide;
-  if (a.counting) {
-    if (wide) tail_variant<true, true>(S, a, b, K, st);
-    else tail_variant<true, false>(S, a, b, K, st);
+  if (a.ordered) {
+    tail_variant<false, kWalkOrd>(S, a, b, K, open_rule(S, a), 0u, st);
+  } else if (a.counting) {
+    if (wide) tail_variant<true, kWalkWide>(S, a, b, K, kOpenNow, 0u, st);
+    else tail_variant<true, kWalkRef>(S, a, b, K, kOpenNow, 0u, st);
   } else {
-    if (wide) tail_variant<false, true>(S, a, b, K, st);
-    else tail_variant<false, false>(S, a, b, K, st);
+    if (wide) tail_variant<false, kWalkWide>(S, a, b, K, kOpenNow, 0u, st);
+    else tail_variant<false, kWalkRef>(S, a, b, K, kOpenNow, 0u, st);
   }
   note_launches(1);
   return cudaGetLastError();
 }
 
-uint32_t walk_lanes() { return walk_grid<false, false>() * (uint32_t)kBlock; }
+bool checks_walks(const DevScene& S, const FrameArgs& a) { return a.ordered && open_rule(S, a) == kOpenCheck; }
+
+cudaError_t launch_verify(const DevScene& S, const RenderBuffers& b, uint32_t list, cudaStream_t st) {
+  const cudaError_t e = cap_launchable(k_verify);
+  if (e != cudaSuccess) return e;
+  k_verify<<<sm_count(), kCapThreads, sizeof(CapShared), st>>>(S, b, list);
+  note_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_tail_again(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K,
+                              cudaStream_t st) {
+  tail_variant<false, kWalkOrd>(S, a, b, K, kOpenNow, 1u, st);
+  note_launches(1);
+  return cudaGetLastError();
+}
+
+uint32_t walk_lanes() {
+  return std::max(walk_grid<false, kWalkRef>(), walk_grid<false, kWalkOrd>()) * (uint32_t)kBlock;
+}
 
 void prepare_launches() {
-  walk_grid<false, false>();
-  walk_grid<false, true>();
-  walk_grid<true, false>();
-  walk_grid<true, true>();
-  tail_grid<false, false>();
-  tail_grid<false, true>();
-  tail_grid<true, false>();
-  tail_grid<true, true>();
+  walk_grid<false, kWalkRef>();
+  walk_grid<false, kWalkWide>();
+  walk_grid<false, kWalkOrd>();
+  walk_grid<true, kWalkRef>();
+  walk_grid<true, kWalkWide>();
+  tail_grid<false, kWalkRef>();
+  tail_grid<false, kWalkWide>();
+  tail_grid<false, kWalkOrd>();
+  tail_grid<true, kWalkRef>();
+  tail_grid<true, kWalkWide>();
   shade_grid();
 }
 
@@ -1405,6 +1715,13 @@ cudaError_t launch_trace_rays(const DevScene& S, const float* rays, uint32_t n, 
     k_trace_rays<false><<<grid, kBlock, 0, st>>>(S, rays, n, maxDist, eps, cullback, t, tri, w, u, v, nodes,
                                                    trisTested);
   note_launches(1);
+  if (!(nodes && trisTested) && S.ord && S.traversal == 0 && !cullback) {
+    const cudaError_t e = cap_launchable(k_resolve_rays);
+    if (e != cudaSuccess) return e;
+    k_resolve_rays<<<std::min<uint32_t>(grid, (uint32_t)sm_count()), kCapThreads, sizeof(CapShared), st>>>(
+        S, rays, n, maxDist, eps, t, tri, w, u, v);
+    note_launches(1);
+  }
   return cudaGetLastError();
 }
 

@@ -31,6 +31,11 @@ struct DevScene {
   const float4* mats = nullptr;
   const uint32_t* lightTri = nullptr;
   const float4* wide = nullptr;  // collapsed 4-wide tree (wide traversal only)
+  // ordered walk (ordered.h; null: the scene keeps the reference's walk): nodes of 6 float4, leaf
+  // records of 4, the largest origin coordinate
+  const float4* ord = nullptr;
+  const float4* ordLeaf = nullptr;
+  float ordRange = 0.f;
   // material textures (only when the scene has any): texels of every texture,
   // one {first texel, width, height, 0} record per texture, and the three
   // vertex uvs of each triangle in BVH order
@@ -58,6 +63,9 @@ struct DevCounters {
   double errSum;          // adaptive: sum of per-pixel errors
   uint32_t carryN[3];     // extension walks carried out of bounce launch L, in counter L % 3
   uint32_t fetchTail;     // next item handed to a lane by the tail kernel
+  uint32_t openN;         // walks of this launch listed for k_resolve
+  uint32_t checkN[2];     // walks of the bounce launches / the tail kernel recorded for k_verify
+  uint32_t fixN;          // of those, paths to run again
   uint32_t tailAt;        // bounce from which the tail kernel carries the frame's paths, when a shading
                           // launch found fewer live paths than FrameArgs::tailBelow (~0u: no switch)
 };
@@ -103,6 +111,7 @@ struct FrameArgs {
   // (decided on the device from the bounce's path count; 0: the fixed switch
   // bounce alone)
   float tailBelow;
+  uint32_t ordered;  // the walks take the ordered tree (scene, camera and options allow it)
 };
 
 struct RenderBuffers {
@@ -138,6 +147,10 @@ struct RenderBuffers {
   // band, launch L's in buffer L & 1
   float4* carry[2];
   uint32_t carryCap;
+  uint32_t* open;         // a launch's walks listed for k_resolve: at most all of its items
+  float4* check;          // two lists of checkCap records of kCheckF4 float4 for k_verify
+  uint32_t* fix;          // records of paths to run again
+  uint32_t checkCap;
   // per bounce d < connDepth and slot (index d * cap + slot): the connection
   // the path made at bounce d, contribution.xyz and .w = 1 when its walk found
   // it unoccluded, 0 when occluded or none was made; k_fold sums them into the
@@ -148,7 +161,8 @@ struct RenderBuffers {
   uint32_t connDepth;
 };
 constexpr uint32_t kMaxBands = 8;
-constexpr uint32_t kCarryF4 = 14;
+constexpr uint32_t kCarryF4 = 16;
+constexpr uint32_t kCheckF4 = 5;
 
 // wavefront kernels (kernels_wave.cu)
 cudaError_t launch_light_pass(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, cudaStream_t st);
@@ -162,6 +176,14 @@ cudaError_t launch_walk(const DevScene& S, const FrameArgs& a, const RenderBuffe
 // attach: store each continuing path's connection at the path's index (for the tail kernel)
 cudaError_t launch_shade(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, int in, uint32_t launch,
                          bool attach, cudaStream_t st);
+// Walks past the reference's pop bound that the frame takes as they ended
+// (checks_walks: whether it does): launch_verify checks those of the bounce
+// launches (list 0) or the tail kernel (1, after list 0), launch_tail_again
+// runs the paths of the wrong ones again from there.
+bool checks_walks(const DevScene& S, const FrameArgs& a);
+cudaError_t launch_verify(const DevScene& S, const RenderBuffers& b, uint32_t list, cudaStream_t st);
+cudaError_t launch_tail_again(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K,
+                              cudaStream_t st);
 // threads of the persistent walk grid (the most walks one launch can carry)
 uint32_t walk_lanes();
 // the sum of every path of the band (connections, then its end): after the

@@ -383,18 +383,4 @@ struct Walk4 {
   __device__ __forceinline__ bool hit() const { return minT < maxDist; }
 };
 
-// walk type, stack entry type and stack depth of the two traversal orders
-template <bool kWide>
-struct WalkOf {
-  using type = Walk;
-  using Entry = uint32_t;
-  static constexpr int kDepth = 32;
-};
-template <>
-struct WalkOf<true> {
-  using type = Walk4;
-  using Entry = uint2;
-  static constexpr int kDepth = (int)kWideDepth;
-};
-
 }  // namespace gbpt

@@ -116,7 +116,8 @@ typedef struct gbpt_params {
   uint32_t carry_steps;     /* walk steps a bounce launch keeps stepping its last extension walks after
                                its ray queue ran dry before handing the unfinished ones, mid-walk, to the
                                next bounce launch (or the tail kernel), where they finish and are shaded one
-                               bounce behind (0: never; default 64; <= 2^20; the reference-order walk only) */
+                               bounce behind (0: never; default 64; <= 2^20; the reference-order walk only; a visit of
+                               an eight-wide node counts as six steps) */
   float tail_below;         /* live paths, as a fraction of the frame's (band's) camera paths, below which a
                                bounce's shading launch hands the remaining bounces to the tail kernel,
                                decided on the device from the bounce's path count ([0, 1]; 0: tail_from
