@@ -842,7 +842,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
     const bool carrying = a.carrySteps && !wideT;
     const size_t np = (size_t)r->W * r->H;
     const uint32_t nb = adaptive ? 1u : bands_for(r->p.bands, np, carrying);
-    const uint32_t K = std::min(tail_from(D, wideT, r->p.tail_from, np / nb, carrying), D);
+    const uint32_t K = std::min(tail_from(D, wideT, a.ordered != 0, r->p.tail_from, np / nb, carrying), D);
     const bool tailRun = K < D || carrying || a.tailBelow > 0.f;
     auto bounces = [&](const RenderBuffers& rbx, cudaStream_t sx, bool mk) -> gbpt_status {
       int in = 0;
@@ -873,7 +873,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
       if (checks) {
         if (aside)
           CK(cudaStreamWaitEvent(sx, r->evJoin[0], 0));
-        else
+        else if (K > 0)
           CK(launch_verify(S, rbx, 0, sx));
         CK(launch_verify(S, rbx, 1, sx));
         CK(launch_tail_again(S, a, rbx, K, sx));

@@ -55,6 +55,17 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
   return m;
 }
 
+// Lanes of a warp that take paths when n of them meet `warps` resident warps:
+// a small frame's paths are spread over a quarter of the warps instead of
+// filling the first few, so that a warp waits for the longest of fewer walks
+// and more warps hide each other's latency.  Cornell 64x64 pass: full warps
+// 0.224 ms, spread over all warps 0.194, half 0.197, a quarter 0.199, an eighth
+// 0.206; at 256x256 all warps cost 4 %, a quarter nothing.
+__device__ __forceinline__ uint32_t path_lanes(uint32_t n, uint32_t warps) {
+  const uint32_t q = max(warps / 4u, 1u), w = max((n + q - 1u) / q, 1u);
+  return w >= 32u ? 0xffffffffu : (1u << w) - 1u;
+}
+
 struct Mat {
   f3 diff, emis;
   float trans, spec, metal, rough;
@@ -1005,17 +1016,18 @@ __global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, Ren
   uint32_t mode = kIdle;
   bool drained = false, resumed = false;
   uint32_t extRays = 0, shRays = 0, nnE = 0, ntE = 0, nnS = 0, ntS = 0;
+  const uint32_t lanes = path_lanes(total, gridDim.x * (kBlock / 32));
   for (;;) {
-    const uint32_t idle = __ballot_sync(0xffffffffu, mode == kIdle);
-    if (idle == 0xffffffffu && drained) break;
+    const uint32_t idle = __ballot_sync(0xffffffffu, mode == kIdle) & lanes;
+    if (idle == lanes && drained) break;
     if constexpr (kKind == kWalkOrd) w.stop_long();
-    if (!drained && (idle == 0xffffffffu || __popc(idle) >= kRefill)) {
+    if (!drained && (idle == lanes || __popc(idle) >= kRefill)) {
       const uint32_t cnt = __popc(idle);
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(&b.ctr->fetchTail, cnt);
       base = __shfl_sync(0xffffffffu, base, 0);
       if (base + cnt >= total) drained = true;
-      if (mode == kIdle) {
+      if ((idle >> lane) & 1u) {
         const uint32_t j = base + __popc(idle & lanemask_lt());
         if (j >= n && j < total) {  // a carried walk: resume it where it stopped
           const float4* r = carried + (size_t)(j - n) * kCarryF4;
@@ -1615,8 +1627,17 @@ void prepare_launches() {
   shade_grid();
 }
 
-uint32_t tail_from(uint32_t eyeDepth, bool wide, int32_t requested, size_t paths, bool carrying) {
-  // default while carrying (reference order): a frame with fewer camera paths
+uint32_t tail_from(uint32_t eyeDepth, bool wide, bool ordered, int32_t requested, size_t paths, bool carrying) {
+  // default for the ordered walk while carrying: a frame with fewer camera paths
+  // than the tail grid has lanes (116,736) runs in the tail kernel alone, a larger
+  // one hands over at bounce D/2 when D > 6, else never.  Measured (ms per case;
+  // first bounce in the tail kernel): Cornell 64x64 pass, D = 8: 0 0.224, 1 0.245,
+  // 2 0.262, 4 0.292; Cornell 256x256 x 16: 0 3.96, 2 4.25, 3 4.16, 8 4.64;
+  // unidirectional 333x217 x 8, D = 10: 0 4.76, 1 5.16, 2 5.49, 5 6.43; 500x375
+  // binary, D = 6: 0 9.90, 3 9.81, none 10.0; interior 1024x768, D = 10: 0 3.72, 4
+  // 3.04, 5 2.90, 6 2.87, none 2.98; hall 1280x720, D = 5: 0 4.10, 4 3.20, none 3.11.
+  //
+  // default of the node-by-node walk while carrying: a frame with fewer camera paths
   // than the walk grid has lanes hands its paths to the tail kernel from bounce
   // 2 on, a larger one from bounce D/2 when D > 6, else never.  Measured with
   // carrying (Mpaths/s; the walk grid then had 194,560 lanes, now 155,648):
@@ -1642,7 +1663,8 @@ uint32_t tail_from(uint32_t eyeDepth, bool wide, int32_t requested, size_t paths
   }();
   if (requested >= 0) return (uint32_t)requested;
   if (v == -2 && carrying) {
-    if (paths < walk_lanes()) return std::min(eyeDepth, 2u);
+    if (ordered && paths < (size_t)tail_grid<false, kWalkOrd>() * kBlock) return 0u;
+    if (!ordered && paths < walk_lanes()) return std::min(eyeDepth, 2u);
     return eyeDepth > 6 ? eyeDepth / 2 : eyeDepth;
   }
   if (v == -2) return eyeDepth > 6 ? eyeDepth / 2 - (wide ? 0u : 1u) : eyeDepth;

@@ -253,7 +253,6 @@ struct OrdWalk {
     gB ^= bit << 24;
     if (gB >> 24) stack[sp++] = make_uint2(gA, gB);
     visit(S, node);
-    pop(stack);
   }
 
   // a walk far past the cap ends here: resolve_capped() answers
@@ -272,11 +271,11 @@ struct OrdWalk {
       gB = 0u;
       sp = 0;
     }
-    pop(stack);
   }
 
   // One iteration of a lone thread; true when the walk is over.
   __device__ __forceinline__ bool step(const DevScene& S, uint2* stack) {
+    pop(stack);
     if (wants_node()) go_node(S, stack);
     if (wants_leaf()) go_leaf(S, stack);
     stop_long();
@@ -289,7 +288,10 @@ struct OrdWalk {
   // lane's walk is over.  (Leaves held back until 8, 16 or 24 lanes have one:
   // hall frame 2.91 -> 2.96, 3.13, 3.65 ms.)
   __device__ __forceinline__ bool step_warp(const DevScene& S, uint2* stack, bool has) {
-    if (has && wants_node()) go_node(S, stack);
+    if (has) {
+      pop(stack);
+      if (wants_node()) go_node(S, stack);
+    }
     __syncwarp();
     if (has && wants_leaf()) go_leaf(S, stack);
     __syncwarp();
