@@ -335,6 +335,7 @@ struct gbpt_renderer {
   cudaStream_t stBand[kMaxBands] = {};
   cudaEvent_t evFork = nullptr, evJoin[kMaxBands] = {};
   uint32_t lastBands = 1;
+  bool refWalk = false;  // this sequence's lists of walks past the pop bound ran full: node-by-node walk
   // window of a larger image (gbpt_renderer_set_window); the whole image by default
   uint32_t winX0 = 0, winY0 = 0, fullW = 0, fullH = 0;
   // frames issued as CUDA graphs (plain and PTSC modes): executable graphs
@@ -488,7 +489,8 @@ RenderBuffers band_buffers(const RenderBuffers& rb, uint32_t b, uint32_t k, size
   x.carry[0] = rb.carry[0] + c0 * kCarryF4;
   x.carry[1] = rb.carry[1] + c0 * kCarryF4;
   x.carryCap = (uint32_t)(c1 - c0);
-  x.open += 2 * p0 + c0;
+  x.openCap = rb.openCap / k;
+  x.open += (size_t)b * x.openCap;
   x.checkCap = rb.checkCap / k;
   x.check += (size_t)b * x.checkCap * 2 * kCheckF4;
   x.fix += (size_t)b * x.checkCap * 2;
@@ -497,16 +499,17 @@ RenderBuffers band_buffers(const RenderBuffers& rb, uint32_t b, uint32_t k, size
 
 }  // namespace
 
-// records for k_verify per list: about one walk in 5,000 needs one; a list that
-// is full costs the walk the reference's own
-static uint32_t check_cap(size_t np) { return (uint32_t)std::max<size_t>(np / 64, 256); }
+// walks listed for k_resolve and records for k_verify, per list: the hall has
+// about one per thousand pixels and frame; a walk that finds its list full
+// takes the reference's walk on the spot
+static uint32_t check_cap(size_t np) { return (uint32_t)std::max<size_t>(np / 256, 256); }
 
 uint64_t gbpt::renderer_bytes(uint32_t W, uint32_t H, const gbpt_params& p) {
   const size_t np = (size_t)W * H;
   const uint32_t cacheCap = std::max(1u, p.light_paths * (1 + p.light_depth_max));
-  return np * (128 + 16 + 96 + 16 + 48 + 16 + 8 + 8) + np * (12 * 10 + 4 * 2 + 4 * 5) + (size_t)cacheCap * 192 +
-         std::max<size_t>(std::min<size_t>(np, walk_lanes()), 256) * (2 * kCarryF4 * 16 + 16 + 4) +
-         (size_t)check_cap(np) * 2 * (kCheckF4 * 16 + 4) +
+  return np * (128 + 16 + 96 + 16 + 48 + 16 + 8) + np * (12 * 10 + 4 * 2 + 4 * 5) + (size_t)cacheCap * 192 +
+         std::max<size_t>(std::min<size_t>(np, walk_lanes()), 256) * (2 * kCarryF4 * 16 + 16) +
+         (size_t)check_cap(np) * (2 * (kCheckF4 * 16 + 4) + 4) +
          np * 16 * (std::max(std::max(p.eye_depth_max, p.pt_depth_max), 2u) - 1);
 }
 
@@ -546,8 +549,8 @@ gbpt_status ensure_alloc(gbpt_renderer* r) {
   CK(dalloc(&r->rb.cache[1], (size_t)cacheCap * 6));
   CK(dalloc(&r->rb.carry[0], (size_t)r->rb.carryCap * kCarryF4));
   CK(dalloc(&r->rb.carry[1], (size_t)r->rb.carryCap * kCarryF4));
-  CK(dalloc(&r->rb.open, 2 * cap + r->rb.carryCap));  // extension and connection rays, resumed walks
-  r->rb.checkCap = check_cap(cap);
+  r->rb.checkCap = r->rb.openCap = check_cap(cap);
+  CK(dalloc(&r->rb.open, r->rb.openCap));
   CK(dalloc(&r->rb.check, (size_t)r->rb.checkCap * 2 * kCheckF4));
   CK(dalloc(&r->rb.fix, (size_t)r->rb.checkCap * 2));
   CK(dalloc(&r->rb.ctr, kMaxBands));
@@ -692,6 +695,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
   }
   bool same = r->started && r->sceneVersion == s->version && std::memcmp(basis9, r->camBasis, sizeof(basis9)) == 0;
   r->frame = same ? r->frame + 1 : 0;
+  if (!same) r->refWalk = false;
   if (!same) r->epoch++;  // light passes made ahead for the old sequence are stale
   std::memcpy(r->camBasis, basis9, sizeof(basis9));
   r->started = true;
@@ -749,7 +753,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
   const DevScene& S = s->dev;
   // the ordered walk answers as the reference's but does not count its pops,
   // and is exact for origins within the scene's range
-  a.ordered = S.ord && S.traversal == 0 && !a.counting && std::fabs(cam->pos[0]) <= S.ordRange &&
+  a.ordered = S.ord && S.traversal == 0 && !a.counting && !r->refWalk && std::fabs(cam->pos[0]) <= S.ordRange &&
               std::fabs(cam->pos[1]) <= S.ordRange && std::fabs(cam->pos[2]) <= S.ordRange;
   cudaStream_t st = r->st;
   // filter-only mode: frames past "Render Iteration" trace nothing and only
@@ -876,7 +880,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
         else if (K > 0)
           CK(launch_verify(S, rbx, 0, sx));
         CK(launch_verify(S, rbx, 1, sx));
-        CK(launch_tail_again(S, a, rbx, K, sx));
+        CK(launch_again(S, a, rbx, sx));
       }
       CK(launch_fold(rbx, sx));
       return GBPT_OK;
@@ -1065,6 +1069,8 @@ gbpt_status render_impl(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam,
     stt = read_ctr(r, &c);
     if (stt != GBPT_OK) return stt;
     flags = c.errFlags;
+    // most walks of this view run out of pops: the node-by-node walk is the faster one
+    if (c.checkN[0] > r->rb.checkCap || c.checkN[1] > r->rb.checkCap) r->refWalk = true;
     if (flags) {
       for (uint32_t b = 0; b < kMaxBands; b++) CK(cudaMemsetAsync(&r->rb.ctr[b].errFlags, 0, 4, r->st));
       CK(cudaStreamSynchronize(r->st));

@@ -27,6 +27,7 @@
 // waits on a count.
 #include <algorithm>
 #include <atomic>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdlib>
@@ -247,14 +248,23 @@ __device__ __forceinline__ LV load_lv(const float4* c) {
 // out exactly as the reference's stable remove_if does: a surviving path's
 // position in the stream equals the number of surviving paths with a lower
 // index, i.e. an exclusive scan of the "alive" flags.
-template <bool kOrdered>
+//
+// kLanes == 8: eight lanes a path (coop_walk) in a cluster of kLightBlocks
+// blocks, whose counts go through distributed shared memory.  The pass is a
+// chain of at most lightDepth + 1 walks whatever the number of paths, so only
+// latency counts: hall 0.62 ms with a lane a path in one block, 0.47 with eight
+// lanes a path in one block, whose 32 warps share four schedulers.
+constexpr uint32_t kLightBlocks = 8;
+template <int kLanes, bool kOrdered>
 __global__ void __launch_bounds__(1024) k_light(DevScene S, FrameArgs a, float4* cache, uint32_t cacheCap,
                                                 DevCounters* ctr) {
   using namespace gb;
-  __shared__ uint32_t warpCnt[32];
-  const uint32_t x = threadIdx.x;
+  __shared__ uint32_t warpCnt[32], openN, blockCnt[2][kLightBlocks];
+  extern __shared__ float4 capMem[];
+  const uint32_t x = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+  const bool first = threadIdx.x % kLanes == 0;  // the path's lane that writes
   const uint32_t NL = a.lightPaths;
-  const uint32_t lane = x & 31, warp = x >> 5, nWarps = (blockDim.x + 31) >> 5;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nWarps = (blockDim.x + 31) >> 5;
   bool alive = (x < NL) && (S.lightN > 0);
   f3 orig = mk(0.f, 0.f, 0.f), dir = orig, outMul = mk(1.f, 1.f, 1.f), sample = orig;
   uint32_t depth = 0;
@@ -284,13 +294,14 @@ __global__ void __launch_bounds__(1024) k_light(DevScene S, FrameArgs a, float4*
     v.spec = m.spec;
     v.metal = m.metal;
     v.rough = m.rough;
-    store_lv(cache + 6 * (size_t)x, v);
+    if (first) store_lv(cache + 6 * (size_t)x, v);
   }
   uint32_t size = (S.lightN > 0) ? NL : 0;
   __syncthreads();
-  for (;;) {
-    uint32_t bal = __ballot_sync(0xffffffffu, alive);
+  for (uint32_t round = 0;; round++) {
+    uint32_t bal = __ballot_sync(0xffffffffu, alive && first);
     if (lane == 0) warpCnt[warp] = __popc(bal);
+    if (threadIdx.x == 0) openN = 0;
     __syncthreads();
     uint32_t before = 0, total = 0;
     for (uint32_t w = 0; w < nWarps; w++) {
@@ -298,25 +309,73 @@ __global__ void __launch_bounds__(1024) k_light(DevScene S, FrameArgs a, float4*
       if (w < warp) before += c;
       total += c;
     }
-    __syncthreads();
+    if constexpr (kLanes > 1) {  // the other blocks' counts (two sets: one is read while the next is written)
+      auto cluster = cooperative_groups::this_cluster();
+      uint32_t* cnt = blockCnt[round & 1u];
+      if (threadIdx.x < kLightBlocks) cluster.map_shared_rank(cnt, threadIdx.x)[blockIdx.x] = total;
+      cluster.sync();
+      total = 0;
+      for (uint32_t k = 0; k < kLightBlocks; k++) {
+        if (k < blockIdx.x) before += cnt[k];
+        total += cnt[k];
+      }
+    } else {
+      __syncthreads();
+    }
     if (total == 0) break;
+    TraceHit h;
+    bool hit = false;
+    if constexpr (kLanes > 1) {  // every lane of the block takes part
+      OrdWalk w;
+      uint2 stack[kOrdStack];
+      w.any = false;
+      w.eps = kBias;
+      w.init(S, orig, dir, kInf);
+      coop_walk(S, w, stack, alive);
+      hit = alive && w.hit();
+      h.t = w.minT, h.tri = w.best, h.u = w.bu, h.v = w.bv;
+      // walks past the pop bound, one after another by the block
+      CapShared& c = *reinterpret_cast<CapShared*>(capMem);
+      const bool open = alive && w.capped();
+      uint32_t turn = open && first ? atomicAdd(&openN, 1u) : 0u;
+      turn = __shfl_sync(0xffffffffu, turn, (int)(lane & ~(uint32_t)(kLanes - 1)));
+      __syncthreads();
+      const uint32_t n = openN;
+      for (uint32_t k = 0; k < n; k++) {
+        __syncthreads();
+        if (open && first && turn == k) {
+          c.hit[0] = st4(orig, 0.f);
+          c.hit[1] = st4(dir, 0.f);
+        }
+        __syncthreads();
+        const f3 o = ld3(c.hit[0]), d = ld3(c.hit[1]);
+        resolve_capped(S, c, o, d, kInf, kBias, false);
+        __syncthreads();
+        if (open && turn == k) {
+          const float4 q = c.answer;
+          hit = c.found != 0u;
+          h.t = q.x, h.tri = __float_as_uint(q.y), h.u = q.z, h.v = q.w;
+        }
+      }
+    }
     if (alive) {
-      uint32_t slot = size + before + __popc(bal & lanemask_lt());
+      uint32_t slot = size + before + __popc(bal & ((1u << (lane & ~(uint32_t)(kLanes - 1))) - 1u));
       if (slot >= cacheCap) {
         atomicOr(&ctr->errFlags, 1u);
         alive = false;
       } else {
         float4* cs = cache + 6 * (size_t)slot;
-        TraceHit h;
-        uint32_t nn = 0, nt = 0;
-        bool hit;
-        if constexpr (kOrdered)
-          hit = trace_ord(S, orig, dir, kInf, kBias, h);
-        else
-          hit = trace_ref<false, false>(S, orig, dir, kInf, kBias, false, h, nn, nt);
+        if constexpr (kLanes == 1) {
+          uint32_t nn = 0, nt = 0;
+          if constexpr (kOrdered)
+            hit = trace_ord(S, orig, dir, kInf, kBias, h);
+          else
+            hit = trace_ref<false, false>(S, orig, dir, kInf, kBias, false, h, nn, nt);
+        }
         if (!hit) {
           const float4* home = cache + 6 * (size_t)x;  // :358-362
-          for (int k = 0; k < 6; k++) cs[k] = home[k];
+          if (first)
+            for (int k = 0; k < 6; k++) cs[k] = home[k];
           alive = false;
         } else {
           float u[8];
@@ -336,7 +395,7 @@ __global__ void __launch_bounds__(1024) k_light(DevScene S, FrameArgs a, float4*
           v.spec = m.spec;
           v.metal = m.metal;
           v.rough = m.rough;
-          store_lv(cs, v);
+          if (first) store_lv(cs, v);
           sample = m.emis + vmul(sample, B.lmt);
           float contrib = length(outMul) * length(B.lmt);
           if (length(m.emis) > 0.f) contrib = 0.f;
@@ -354,7 +413,7 @@ __global__ void __launch_bounds__(1024) k_light(DevScene S, FrameArgs a, float4*
     size += total;
     __syncthreads();
   }
-  if (x == 0) ctr->cacheSize[a.cacheSel] = size;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctr->cacheSize[a.cacheSel] = size;
 }
 
 // ---------------------------------------------------------------------------
@@ -729,8 +788,15 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(DevScene S, RenderBuffers b,
         bool open = false;
         if constexpr (kKind == kWalkOrd) {
           if (w.capped()) {
-            open = later == kOpenList;
-            bool now = later == kOpenNow || w.bound >= kPopStop;  // an unfinished walk has no answer to take
+            bool now = later == kOpenNow;
+            if (later == kOpenList) {
+              const uint32_t k = atomicAdd(&b.ctr->openN, 1u);
+              open = k < b.openCap;
+              now = !open;
+              if (open) b.open[k] = item | (res ? kOpenCarried : any ? kOpenShadow : 0u);
+            } else if (later == kOpenCheck) {
+              now = w.bound >= kPopStop;  // an unfinished walk has no answer to take
+            }
             if (later == kOpenCheck && !now) {
               const float4* q = res ? prev + (size_t)item * kCarryF4 : any ? sh + 3 * (size_t)item : wv.o + item;
               const size_t st = (res || any) ? 1 : (size_t)(wv.d - wv.o);
@@ -738,7 +804,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(DevScene S, RenderBuffers b,
                                 any ? make_float4(0.f, 0.f, 0.f, __uint_as_float(kShadowRec)) : q[3 * st],
                                 make_float4(w.hit() ? w.minT : -1.f, __uint_as_float(w.best), w.bu, w.bv));
             }
-            if (!open && now) {
+            if (now) {
               TraceHit h;
               uint32_t nn = 0, nt = 0;
               const float far = any ? (res ? prev + (size_t)item * kCarryF4 : sh + 3 * (size_t)item)[1].w : gb::kInf;
@@ -748,7 +814,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(DevScene S, RenderBuffers b,
           }
         }
         if (open) {
-          b.open[atomicAdd(&b.ctr->openN, 1u)] = item | (res ? kOpenCarried : any ? kOpenShadow : 0u);
+          // k_resolve stores its answer
         } else if (any) {
           const float4* q = res ? prev + (size_t)item * kCarryF4 : sh + 3 * (size_t)item;
           if (!w.hit()) connection_reached(b, bilat, q[0], q[2]);  // unoccluded: it counts (:716-721)
@@ -988,21 +1054,30 @@ enum : uint32_t { kIdle = 0, kPathExt = 1, kPathShadow = 2 };
 // 192.7.  Three CTAs per SM (80 registers, some spill) against two (116
 // registers): interior 167.0 -> 170.0, Cornell 195.6 -> 193.6 Mpaths/s; four
 // (64 registers): hall 195.9 -> 194.6, Cornell 190.4 -> 183.1.
+// The ordered walk's tail: two CTAs per SM (128 registers, no spill) against
+// three (80, 390 bytes of spill stores) and four: Cornell 256x256 image 3.61 /
+// 3.99 / 4.50 ms, unidirectional 333x217 image 4.46 / 4.86 / 5.34, hall pass 2.94 /
+// 2.97 / 2.99; 12 and 24 steps between refill checks within 2 % of 16.
+template <int kKind>
+__host__ __device__ constexpr int tail_ctas() {
+  return kKind == kWalkOrd ? 2 : 3;
+}
 template <int kKind>
 __host__ __device__ constexpr int tail_steps() {
   return kKind == kWalkOrd ? 16 : 64;
 }
 
-template <bool kCount, int kKind>
-__global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, RenderBuffers b, uint32_t K,
-                                                   uint32_t kRefill, uint32_t later, uint32_t again) {
+// kLater: what becomes of walks past the pop bound (kOpenNow etc.), fixed at
+// compile time so that a kernel holds only its own case's code.
+template <bool kCount, int kKind, uint32_t kLater = kOpenNow>
+__global__ void __launch_bounds__(kBlock, tail_ctas<kKind>()) k_tail(DevScene S, FrameArgs a, RenderBuffers b, uint32_t K,
+                                                   uint32_t kRefill) {
   // t: the launch the bounce launches stopped before (the device switch or K)
   const uint32_t t = min(b.ctr->tailAt, K);
   const int in = (int)(t & 1u);
   const int shIn = t > 0 ? (int)((t - 1) & 1u) : -1;
-  // again: only the paths whose recorded answer k_verify corrected, from there on
-  const uint32_t n = again ? 0u : b.ctr->wave[in];
-  const uint32_t nCarry = again ? b.ctr->fixN : t > 0 ? carried_of(b, t - 1) : 0u;
+  const uint32_t n = b.ctr->wave[in];
+  const uint32_t nCarry = t > 0 ? carried_of(b, t - 1) : 0u;
   const float4* carried = b.carry[(t + 1) & 1u];  // launch t - 1's
   const uint32_t total = n + nCarry;
   const uint32_t cacheSize = b.lctr->cacheSize[a.cacheSel];
@@ -1032,32 +1107,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, Ren
         if (j >= n && j < total) {  // a carried walk: resume it where it stopped
           const float4* r = carried + (size_t)(j - n) * kCarryF4;
           resumed = true;
-          if (kKind == kWalkOrd && again) {
-            const uint32_t k = j - n;
-            r = b.check + (size_t)b.fix[k] * kCheckF4;
-            io.o = r[0];
-            io.d = r[1];
-            io.t = r[2];
-            io.s = r[3];
-            mode = kPathExt;
-            // a path corrected at an earlier bounce as well starts there
-            for (uint32_t m = 0; m < nCarry; m++) {
-              const float4* q = b.check + (size_t)b.fix[m] * kCheckF4;
-              if (__float_as_uint(q[0].w) == __float_as_uint(io.o.w) &&
-                  __float_as_uint(q[3].w) < __float_as_uint(io.s.w))
-                mode = kIdle;
-            }
-            if constexpr (kKind == kWalkOrd) {
-              start_walk<kKind>(S, w, ld3(io.o), ld3(io.d), gb::kInf, false, stack);
-              w.gB = 0u;  // over, with the corrected answer
-              w.settle(r[4].x >= 0.f, r[4]);
-            }
-            resumed = mode != kIdle;
-            if (a.gbuffer && resumed && __float_as_uint(io.s.w) == 0u) {  // as k_camera leaves them
-              float4* g = b.gbuf + 3 * (size_t)__float_as_uint(io.o.w);
-              g[0] = g[1] = g[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-          } else if constexpr (kKind != kWalkWide) {
+          if constexpr (kKind != kWalkWide) {
             if (resume_walk(S, r, w, stack)) {  // a connection alone, without its path
               io.shA = r[0];
               io.shB = r[1];
@@ -1103,10 +1153,21 @@ __global__ void __launch_bounds__(kBlock, 3) k_tail(DevScene S, FrameArgs a, Ren
       if (mode == kIdle) continue;
       if (done && w.capped()) {
         const float4 got = make_float4(w.hit() ? w.minT : -1.f, __uint_as_float(w.best), w.bu, w.bv);
+        // an extension walk of a mode whose shading cannot be undone waits for
+        // its answer (t -2: to be run on from there whatever it is); so would the
+        // connection whose direct-light sample the next shading reads
+        const bool wait = kLater == kOpenList && !anyHit;
+        const bool direct = kLater == kOpenList && anyHit && a.bilat && __float_as_uint(io.shC.w) == 0u;
         const bool noted =
-            later == kOpenCheck && w.bound < kPopStop &&
+            kLater != kOpenNow && !direct && (wait || w.bound < kPopStop) &&
             (anyHit ? note_check(b, 1, io.shA, io.shB, io.shC, make_float4(0.f, 0.f, 0.f, __uint_as_float(kShadowRec)), got)
-                    : note_check(b, 1, io.o, io.d, io.t, io.s, got));
+                    : note_check(b, 1, io.o, io.d, io.t, io.s, wait ? make_float4(-2.f, 0.f, 0.f, 0.f) : got));
+        if (noted && wait) {
+          if (!resumed) extRays++;
+          resumed = false;
+          mode = kIdle;
+          continue;
+        }
         if (!noted) {
           TraceHit h;
           uint32_t nn = 0, nt = 0;
@@ -1170,7 +1231,7 @@ __global__ void __launch_bounds__(kCapThreads) k_resolve(DevScene S, RenderBuffe
   extern __shared__ float4 capMem[];
   CapShared& c = *reinterpret_cast<CapShared*>(capMem);
   if (b.ctr->tailAt <= launch) return;
-  const uint32_t n = b.ctr->openN, nE = (in >= 0) ? b.ctr->wave[in] : 0u;
+  const uint32_t n = min(b.ctr->openN, b.openCap), nE = (in >= 0) ? b.ctr->wave[in] : 0u;
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
     const uint32_t code = b.open[i], item = code & kOpenItem;
     const bool res = (code & kOpenCarried) != 0u;
@@ -1192,8 +1253,8 @@ __global__ void __launch_bounds__(kCapThreads) k_resolve(DevScene S, RenderBuffe
 
 // Checks the recorded answers of one list, one block each.  A connection's
 // entry is set right here; a path whose closest hit was another gets its
-// record's answer corrected and joins the list the tail kernel runs again from
-// that bounce, which rewrites everything the path wrote from there on (its
+// record's answer corrected and joins the list k_again runs from that bounce,
+// which rewrites everything the path wrote from there on (its
 // connection entries, its end, its first-hit planes).  The bounce launches'
 // list is checked beside the tail kernel.
 __global__ void __launch_bounds__(kCapThreads) k_verify(DevScene S, RenderBuffers b, uint32_t list) {
@@ -1214,12 +1275,86 @@ __global__ void __launch_bounds__(kCapThreads) k_verify(DevScene S, RenderBuffer
         const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
         b.conn[(size_t)__float_as_uint(C.w) * b.cap + __float_as_uint(A.w)] = hit ? none : make_float4(C.x, C.y, C.z, 1.f);
       }
-    } else if (hit != was || (hit && (c.answer.x != got.x || __float_as_uint(c.answer.y) != __float_as_uint(got.y)))) {
+    } else if (got.x == -2.f || hit != was || (hit && (c.answer.x != got.x || __float_as_uint(c.answer.y) != __float_as_uint(got.y)))) {
       r[4] = hit ? c.answer : make_float4(-1.f, 0.f, 0.f, 0.f);
       b.fix[atomicAdd(&b.ctr->fixN, 1u)] = rec;
     }
   }
-  if (list == 1u && blockIdx.x == 0 && threadIdx.x == 0) b.ctr->fetchTail = 0;  // for the tail kernel's second run
+}
+
+// The paths k_verify listed, from the bounce of their record on with its
+// answer, one block each: few and alone on the GPU, so their latency counts.
+// Walks run eight lanes a ray (coop_walk, every group the same ray), those past
+// the pop bound are resolved by the block at once; one thread shades.
+__global__ void __launch_bounds__(kCapThreads) k_again(DevScene S, FrameArgs a, RenderBuffers b) {
+  extern __shared__ float4 capMem[];
+  CapShared& c = *reinterpret_cast<CapShared*>(capMem);
+  __shared__ float4 path[7];
+  __shared__ uint32_t flags;
+  const uint32_t n = b.ctr->fixN;
+  const uint32_t cacheSize = b.lctr->cacheSize[a.cacheSel];
+  const float4* __restrict__ cache = b.cache[a.cacheSel];
+  uint32_t extRays = 0, shRays = 0;
+  // the answer of one ray, for every thread; (-1, ...) on a miss
+  auto walk = [&](float4 o, float4 d, float far, bool any) {
+    OrdWalk w;
+    uint2 stack[kOrdStack];
+    w.any = any;
+    w.eps = gb::kBias;
+    w.init(S, ld3(o), ld3(d), far);
+    coop_walk(S, w, stack, true);
+    if (!w.capped()) return w.hit() ? make_float4(w.minT, __uint_as_float(w.best), w.bu, w.bv)
+                                    : make_float4(-1.f, 0.f, 0.f, 0.f);
+    resolve_capped(S, c, ld3(o), ld3(d), far, gb::kBias, any);
+    __syncthreads();
+    const float4 h = c.found ? c.answer : make_float4(-1.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    return h;
+  };
+  for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) {
+    const float4* r = b.check + (size_t)b.fix[k] * kCheckF4;
+    PathIO io;
+    io.o = r[0];
+    io.d = r[1];
+    io.t = r[2];
+    io.s = r[3];
+    float4 h = r[4];
+    bool skip = false;  // a path corrected at an earlier bounce as well starts there
+    for (uint32_t m = 0; m < n; m++) {
+      const float4* q = b.check + (size_t)b.fix[m] * kCheckF4;
+      skip |= __float_as_uint(q[0].w) == __float_as_uint(io.o.w) && __float_as_uint(q[3].w) < __float_as_uint(io.s.w);
+    }
+    if (skip) continue;  // block-uniform
+    if (a.gbuffer && threadIdx.x == 0 && __float_as_uint(io.s.w) == 0u) {  // as k_camera leaves them
+      float4* g = b.gbuf + 3 * (size_t)__float_as_uint(io.o.w);
+      g[0] = g[1] = g[2] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (;;) {
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        shade_path(S, a, b, cache, cacheSize, __float_as_uint(io.s.w), h, io);
+        path[0] = io.o, path[1] = io.d, path[2] = io.t, path[3] = io.s;
+        path[4] = io.shA, path[5] = io.shB, path[6] = io.shC;
+        flags = (io.cont ? 1u : 0u) | (io.conn ? 2u : 0u);
+      }
+      __syncthreads();
+      io.o = path[0], io.d = path[1], io.t = path[2], io.s = path[3];
+      const uint32_t f = flags;
+      if (!(f & 1u)) break;
+      if (f & 2u) {
+        const float4 A = path[4], B = path[5], C = path[6];
+        const float4 q = walk(A, B, B.w, true);
+        if (threadIdx.x == 0 && q.x < 0.f) connection_reached(b, a.bilat, A, C);
+        shRays++;
+      }
+      h = walk(io.o, io.d, gb::kInf, false);
+      extRays++;
+    }
+  }
+  if (threadIdx.x == 0 && extRays) {
+    atomicAdd(&b.ctr->rays, (unsigned long long)(extRays + shRays));
+    atomicAdd(&b.ctr->shadowRays, (unsigned long long)shRays);
+  }
 }
 
 // ... and of caller-supplied rays (k_trace_rays marks them with triangle -2):
@@ -1399,6 +1534,9 @@ template <bool kCount>
 __global__ void k_trace_rays(DevScene S, const float* rays, uint32_t n, float maxDist, float eps, int cullback,
                              float* t, int32_t* tri, float* w, float* u, float* v, uint32_t* nodes,
                              uint32_t* trisTested) {
+  __shared__ uint32_t openN;
+  if (threadIdx.x == 0) openN = 0;
+  __syncthreads();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float* r = rays + 6 * (size_t)i;
@@ -1419,10 +1557,15 @@ __global__ void k_trace_rays(DevScene S, const float* rays, uint32_t n, float ma
     h.v = wk.bv;
   } else if (!kCount && S.ord && S.traversal == 0 && !cullback) {
     bool open = false;
-    hit = trace_ord(S, mk(r[0], r[1], r[2]), mk(r[3], r[4], r[5]), maxDist, eps, h, &open);
+    const f3 o = mk(r[0], r[1], r[2]), d = mk(r[3], r[4], r[5]);
+    hit = trace_ord(S, o, d, maxDist, eps, h, &open);
     if (open) {
-      tri[i] = -2;  // for k_resolve_rays
-      return;
+      // a few of a block's rays wait for k_resolve_rays, more take the reference's walk
+      if (atomicAdd(&openN, 1u) < 4u) {
+        tri[i] = -2;
+        return;
+      }
+      hit = trace_ref<false, false>(S, o, d, maxDist, eps, false, h, nn, nt);
     }
   } else {
     hit = trace_ref<false, kCount>(S, mk(r[0], r[1], r[2]), mk(r[3], r[4], r[5]), maxDist, eps, cullback != 0, h,
@@ -1479,13 +1622,37 @@ int sm_count() {
   return g_sm;
 }
 
+// opens a kernel for the lists' shared memory
+template <typename Kern>
+cudaError_t cap_launchable(Kern kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CapShared));
+}
+
 cudaError_t launch_light_pass(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, cudaStream_t st) {
   uint32_t threads = ((a.lightPaths + 31) / 32) * 32;
   if (threads == 0) threads = 32;
-  if (a.ordered)
-    k_light<true><<<1, threads, 0, st>>>(S, a, b.cache[a.cacheSel], b.cacheCap, b.ctr);
-  else
-    k_light<false><<<1, threads, 0, st>>>(S, a, b.cache[a.cacheSel], b.cacheCap, b.ctr);
+  float4* cache = b.cache[a.cacheSel];
+  if (a.ordered && threads <= 128) {
+    const cudaError_t e = cap_launchable(k_light<8, true>);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kLightBlocks);
+    cfg.blockDim = dim3(threads * 8 / kLightBlocks);
+    cfg.dynamicSmemBytes = sizeof(CapShared);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kLightBlocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, k_light<8, true>, S, a, cache, b.cacheCap, b.ctr);
+    if (le != cudaSuccess) return le;
+  } else if (a.ordered) {
+    k_light<1, true><<<1, threads, 0, st>>>(S, a, cache, b.cacheCap, b.ctr);
+  } else {
+    k_light<1, false><<<1, threads, 0, st>>>(S, a, cache, b.cacheCap, b.ctr);
+  }
   note_launches(1);
   return cudaGetLastError();
 }
@@ -1503,9 +1670,9 @@ uint32_t walk_grid() {
   return g;
 }
 
-template <bool kCount, int kKind>
+template <bool kCount, int kKind, uint32_t kLater = kOpenNow>
 uint32_t tail_grid() {
-  static uint32_t g = grid_for((const void*)k_tail<kCount, kKind>);
+  static uint32_t g = grid_for((const void*)k_tail<kCount, kKind, kLater>);
   return g;
 }
 
@@ -1529,19 +1696,13 @@ void walk_variant(const DevScene& S, const RenderBuffers& b, int in, int shIn, i
   k_walk<kCount, kKind><<<g, kBlock, 0, st>>>(S, b, in, shIn, shReset, bilat, refill, launch, carrySteps, later);
 }
 
-template <bool kCount, int kKind>
-void tail_variant(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K, uint32_t later,
-                  uint32_t again, cudaStream_t st) {
-  const uint32_t g = persistent_grid(tail_grid<kCount, kKind>(), a.walkCtas);
-  k_tail<kCount, kKind><<<g, kBlock, 0, st>>>(S, a, b, K, walk_refill_for(a.refill, kKind == kWalkWide), later, again);
+template <bool kCount, int kKind, uint32_t kLater = kOpenNow>
+void tail_variant(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K, cudaStream_t st) {
+  const uint32_t g = persistent_grid(tail_grid<kCount, kKind, kLater>(), a.walkCtas);
+  k_tail<kCount, kKind, kLater><<<g, kBlock, 0, st>>>(S, a, b, K, walk_refill_for(a.refill, kKind == kWalkWide));
 }
 
-// one block per SM (its lists take half of an SM's shared memory): opens the
-// kernel for that much once per device context
-template <typename Kern>
-cudaError_t cap_launchable(Kern kern) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CapShared));
-}
+uint32_t cap_grid() { return 4u * (uint32_t)sm_count(); }
 
 // what becomes of walks past the pop bound: a tree of up to 2048 nodes cannot
 // have any; the filter-only mode's direct-light sample and the learned
@@ -1563,7 +1724,7 @@ cudaError_t launch_walk(const DevScene& S, const FrameArgs& a, const RenderBuffe
     if (open_rule(S, a) == kOpenList) {
       const cudaError_t e = cap_launchable(k_resolve);
       if (e != cudaSuccess) return e;
-      k_resolve<<<sm_count(), kCapThreads, sizeof(CapShared), st>>>(S, b, in, shIn, sd, launch);
+      k_resolve<<<cap_grid(), kCapThreads, sizeof(CapShared), st>>>(S, b, in, shIn, sd, launch);
       note_launches(1);
     }
   } else if (a.counting) {
@@ -1580,31 +1741,35 @@ cudaError_t launch_walk(const DevScene& S, const FrameArgs& a, const RenderBuffe
 cudaError_t launch_tail(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K, cudaStream_t st) {
   const bool wide = S.traversal == 1 && S.wide;
   if (a.ordered) {
-    tail_variant<false, kWalkOrd>(S, a, b, K, open_rule(S, a), 0u, st);
+    const uint32_t rule = open_rule(S, a);
+    if (rule == kOpenNow) tail_variant<false, kWalkOrd, kOpenNow>(S, a, b, K, st);
+    else if (rule == kOpenList) tail_variant<false, kWalkOrd, kOpenList>(S, a, b, K, st);
+    else tail_variant<false, kWalkOrd, kOpenCheck>(S, a, b, K, st);
   } else if (a.counting) {
-    if (wide) tail_variant<true, kWalkWide>(S, a, b, K, kOpenNow, 0u, st);
-    else tail_variant<true, kWalkRef>(S, a, b, K, kOpenNow, 0u, st);
+    if (wide) tail_variant<true, kWalkWide>(S, a, b, K, st);
+    else tail_variant<true, kWalkRef>(S, a, b, K, st);
   } else {
-    if (wide) tail_variant<false, kWalkWide>(S, a, b, K, kOpenNow, 0u, st);
-    else tail_variant<false, kWalkRef>(S, a, b, K, kOpenNow, 0u, st);
+    if (wide) tail_variant<false, kWalkWide>(S, a, b, K, st);
+    else tail_variant<false, kWalkRef>(S, a, b, K, st);
   }
   note_launches(1);
   return cudaGetLastError();
 }
 
-bool checks_walks(const DevScene& S, const FrameArgs& a) { return a.ordered && open_rule(S, a) == kOpenCheck; }
+bool checks_walks(const DevScene& S, const FrameArgs& a) { return a.ordered && open_rule(S, a) != kOpenNow; }
 
 cudaError_t launch_verify(const DevScene& S, const RenderBuffers& b, uint32_t list, cudaStream_t st) {
   const cudaError_t e = cap_launchable(k_verify);
   if (e != cudaSuccess) return e;
-  k_verify<<<sm_count(), kCapThreads, sizeof(CapShared), st>>>(S, b, list);
+  k_verify<<<cap_grid(), kCapThreads, sizeof(CapShared), st>>>(S, b, list);
   note_launches(1);
   return cudaGetLastError();
 }
 
-cudaError_t launch_tail_again(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K,
-                              cudaStream_t st) {
-  tail_variant<false, kWalkOrd>(S, a, b, K, kOpenNow, 1u, st);
+cudaError_t launch_again(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, cudaStream_t st) {
+  const cudaError_t e = cap_launchable(k_again);
+  if (e != cudaSuccess) return e;
+  k_again<<<sm_count(), kCapThreads, sizeof(CapShared), st>>>(S, a, b);
   note_launches(1);
   return cudaGetLastError();
 }
@@ -1621,7 +1786,9 @@ void prepare_launches() {
   walk_grid<true, kWalkWide>();
   tail_grid<false, kWalkRef>();
   tail_grid<false, kWalkWide>();
-  tail_grid<false, kWalkOrd>();
+  tail_grid<false, kWalkOrd, kOpenNow>();
+  tail_grid<false, kWalkOrd, kOpenList>();
+  tail_grid<false, kWalkOrd, kOpenCheck>();
   tail_grid<true, kWalkRef>();
   tail_grid<true, kWalkWide>();
   shade_grid();
@@ -1629,13 +1796,13 @@ void prepare_launches() {
 
 uint32_t tail_from(uint32_t eyeDepth, bool wide, bool ordered, int32_t requested, size_t paths, bool carrying) {
   // default for the ordered walk while carrying: a frame with fewer camera paths
-  // than the tail grid has lanes (116,736) runs in the tail kernel alone, a larger
-  // one hands over at bounce D/2 when D > 6, else never.  Measured (ms per case;
-  // first bounce in the tail kernel): Cornell 64x64 pass, D = 8: 0 0.224, 1 0.245,
-  // 2 0.262, 4 0.292; Cornell 256x256 x 16: 0 3.96, 2 4.25, 3 4.16, 8 4.64;
-  // unidirectional 333x217 x 8, D = 10: 0 4.76, 1 5.16, 2 5.49, 5 6.43; 500x375
-  // binary, D = 6: 0 9.90, 3 9.81, none 10.0; interior 1024x768, D = 10: 0 3.72, 4
-  // 3.04, 5 2.90, 6 2.87, none 2.98; hall 1280x720, D = 5: 0 4.10, 4 3.20, none 3.11.
+  // than 1.5 x the tail grid's lanes (116,736) runs in the tail kernel alone, a
+  // larger one hands over at bounce 3D/5 when D > 6, else never.  Measured (ms per
+  // case; first bounce in the tail kernel): Cornell 64x64 pass, D = 8: 0 0.202, 2
+  // 0.231, 4 0.254; Cornell 256x256 x 16: 0 3.62, 2 3.93, 4 4.03, 7 4.36;
+  // unidirectional 333x217 x 8, D = 10: 0 4.49, 2 5.35, 5 6.19; 500x375 binary, D =
+  // 6: 0 10.0, 4 9.40, none 9.64; interior 1024x768, D = 10: 0 4.20, 4 3.06, 5 2.88,
+  // 6 2.80, 7 2.80; hall 1280x720, D = 5: 0 4.59, 4 3.06, none 2.94.
   //
   // default of the node-by-node walk while carrying: a frame with fewer camera paths
   // than the walk grid has lanes hands its paths to the tail kernel from bounce
@@ -1663,9 +1830,9 @@ uint32_t tail_from(uint32_t eyeDepth, bool wide, bool ordered, int32_t requested
   }();
   if (requested >= 0) return (uint32_t)requested;
   if (v == -2 && carrying) {
-    if (ordered && paths < (size_t)tail_grid<false, kWalkOrd>() * kBlock) return 0u;
+    if (ordered && paths < (size_t)tail_grid<false, kWalkOrd>() * kBlock * 3 / 2) return 0u;
     if (!ordered && paths < walk_lanes()) return std::min(eyeDepth, 2u);
-    return eyeDepth > 6 ? eyeDepth / 2 : eyeDepth;
+    return eyeDepth > 6 ? (ordered ? eyeDepth * 3 / 5 : eyeDepth / 2) : eyeDepth;
   }
   if (v == -2) return eyeDepth > 6 ? eyeDepth / 2 - (wide ? 0u : 1u) : eyeDepth;
   return v < 0 ? eyeDepth : (uint32_t)v;
@@ -1740,7 +1907,7 @@ cudaError_t launch_trace_rays(const DevScene& S, const float* rays, uint32_t n, 
   if (!(nodes && trisTested) && S.ord && S.traversal == 0 && !cullback) {
     const cudaError_t e = cap_launchable(k_resolve_rays);
     if (e != cudaSuccess) return e;
-    k_resolve_rays<<<std::min<uint32_t>(grid, (uint32_t)sm_count()), kCapThreads, sizeof(CapShared), st>>>(
+    k_resolve_rays<<<std::min<uint32_t>(grid, cap_grid()), kCapThreads, sizeof(CapShared), st>>>(
         S, rays, n, maxDist, eps, t, tri, w, u, v);
     note_launches(1);
   }

@@ -147,7 +147,8 @@ struct RenderBuffers {
   // band, launch L's in buffer L & 1
   float4* carry[2];
   uint32_t carryCap;
-  uint32_t* open;         // a launch's walks listed for k_resolve: at most all of its items
+  uint32_t* open;         // a launch's walks listed for k_resolve, up to openCap
+  uint32_t openCap;
   float4* check;          // two lists of checkCap records of kCheckF4 float4 for k_verify
   uint32_t* fix;          // records of paths to run again
   uint32_t checkCap;
@@ -182,8 +183,7 @@ cudaError_t launch_shade(const DevScene& S, const FrameArgs& a, const RenderBuff
 // runs the paths of the wrong ones again from there.
 bool checks_walks(const DevScene& S, const FrameArgs& a);
 cudaError_t launch_verify(const DevScene& S, const RenderBuffers& b, uint32_t list, cudaStream_t st);
-cudaError_t launch_tail_again(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K,
-                              cudaStream_t st);
+cudaError_t launch_again(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, cudaStream_t st);
 // threads of the persistent walk grid (the most walks one launch can carry)
 uint32_t walk_lanes();
 // the sum of every path of the band (connections, then its end): after the

@@ -299,6 +299,120 @@ struct OrdWalk {
   }
 };
 
+// The walks of up to four rays run by a warp, eight lanes a ray (group g = lanes
+// 8g .. 8g + 7, all holding the same walk): lane c tests child c of the
+// node and, of the leaves that come next in the order, the one in slot c; hits
+// are then taken in the order.  The same tests on the same values as
+// OrdWalk::visit and leaf.  A lone long walk is a chain of dependent fetches
+// and instructions; this shortens the instructions' part (some 400 an iteration
+// for a single lane) several times over.
+__device__ __forceinline__ void coop_walk(const DevScene& S, OrdWalk& w, uint2* stack, bool live) {
+  using namespace gb;
+  const uint32_t lane = threadIdx.x & 31u, c = lane & 7u, group = lane & 24u;
+  const bool nx = __float_as_int(w.inv.x) < 0, ny = __float_as_int(w.inv.y) < 0, nz = __float_as_int(w.inv.z) < 0;
+  const uint32_t sel = 0x7604u | ((c & 3u) << 4);  // byte c & 3 as in byte_float
+  const bool high = c >= 4u;
+  for (;;) {
+    w.stop_long();
+    if (live) w.pop(stack);
+    if (!__any_sync(0xffffffffu, live && !w.over())) break;
+    const bool node = live && w.wants_node();
+    bool hit = false;
+    uint32_t nextA = w.gA, nextB = w.gB;
+    if (node) {
+      const uint32_t bit = w.next();
+      const uint32_t id = (w.gA & 0xFFFFFFu) + __popc((w.gA >> 24) & (bit - 1u));
+      const float4* r = S.ord + 6 * (size_t)id;
+      float4 A, B, X, Y;
+      ldg_node(r, A, B);
+      ldg_node(r + 2, X, Y);
+      const float4 Z = __ldg(r + 4);
+      w.gB ^= bit << 24;
+      if (w.gB >> 24) stack[w.sp++] = make_uint2(w.gA, w.gB);
+      nextA = __float_as_uint(B.z);
+      nextB = __float_as_uint(B.w);
+      w.bound += 2u * (nextB >> 24);
+      const float ix = w.inv.x * w.scale, iy = w.inv.y * w.scale, iz = w.inv.z * w.scale;
+      const float sx = A.w * ix, sy = B.x * iy, sz = B.y * iz;
+      const float cx = fma_(A.x - w.o.x, ix, -sx), cy = fma_(A.y - w.o.y, iy, -sy), cz = fma_(A.z - w.o.z, iz, -sz);
+      auto plane = [&](float lo, float hi) {
+        return __uint_as_float(__byte_perm(__float_as_uint(high ? hi : lo), 0x3F800000u, sel));
+      };
+      const float lx = plane(X.x, X.y), hx = plane(X.z, X.w), ly = plane(Y.x, Y.y), hy = plane(Y.z, Y.w),
+                  lz = plane(Z.x, Z.y), hz = plane(Z.z, Z.w);
+      const float n = fmax3_(fma_(nx ? hx : lx, sx, cx), fma_(ny ? hy : ly, sy, cy), fma_sat(nz ? hz : lz, sz, cz));
+      const float f = fmin3_(fma_(nx ? lx : hx, sx, cx), fma_(ny ? ly : hy, sy, cy), fma_sat(nz ? lz : hz, sz, cz));
+      hit = n < f;
+    }
+    const uint32_t hits = (__ballot_sync(0xffffffffu, hit) >> group) & 0xFFu;
+    if (node) {
+      w.gA = nextA;
+      w.gB = (nextB & 0xFFFFFFu) | hits << 24;
+      w.pop(stack);
+    }
+    // the leaves before the next inner child
+    const uint32_t m = w.gB >> 24, im = w.gA >> 24, in = m & im;
+    const uint32_t run = live ? m & ((in & (0u - in)) - 1u) & ~im : 0u;
+    if (!__any_sync(0xffffffffu, run != 0u)) continue;
+    bool cand = false;
+    float near = 0.f, rT = 0.f, u = 0.f, v = 0.f;
+    uint32_t id = 0;
+    bool many = false;
+    if ((run >> c) & 1u) {
+      const float4* r = S.ordLeaf + 4 * (size_t)((w.gB & 0xFFFFFFu) + c - __popc(im & ((1u << c) - 1u)));
+      float4 a, b, q, e;
+      ldg_node(r, a, b);
+      ldg_node(r + 2, q, e);
+      id = __float_as_uint(e.w);
+      many = (id & kOrdManyTris) != 0u;
+      const bool box = slab_hit((q.y - w.o.x) * w.inv.x, (e.x - w.o.x) * w.inv.x, (q.z - w.o.y) * w.inv.y,
+                                (e.y - w.o.y) * w.inv.y, (q.w - w.o.z) * w.inv.z, (e.z - w.o.z) * w.inv.z,
+                                __uint_as_float(0x7f800000u), near);
+      const f3 E0 = mk(a.w, b.x, b.y), E1 = mk(b.z, b.w, q.x), de2 = cross(w.d, E1);
+      float div = dot(de2, E0);
+      if (box && !many && !(fabsf(div) < kLtEps9)) {
+        div = rcp_(div);
+        const f3 t = (w.o + w.eps * w.d) - mk(a.x, a.y, a.z), te1 = cross(t, E0);
+        rT = dot(te1, E1) * div;
+        u = dot(de2, t) * div;
+        v = dot(te1, w.d) * div;
+        cand = rT >= 0.f && !(u < 0.f || u > 1.f) && !(v < 0.f || (u + v) > 1.f);
+      }
+    }
+    const uint32_t manyRun = (__ballot_sync(0xffffffffu, many) >> group) & 0xFFu;
+    if (manyRun) {  // leaves of several triangles: the run one leaf after another, by every lane of the group
+      for (uint32_t left = run; left; left &= left - 1u)
+        if (w.gB >> 24) w.go_leaf(S, stack);
+      cand = false;
+    }
+    const bool took = run != 0u && !manyRun;
+    if (took) w.gB ^= run << 24;
+    for (uint32_t from = 0;;) {
+      const uint32_t ok = __ballot_sync(0xffffffffu, cand && c >= from && near < w.minT && rT < w.minT);
+      if (ok == 0u) break;
+      const uint32_t mine = (ok >> group) & 0xFFu;
+      const int src = mine ? (int)group + __ffs((int)mine) - 1 : (int)lane;
+      const float t1 = __shfl_sync(0xffffffffu, rT, src), u1 = __shfl_sync(0xffffffffu, u, src),
+                  v1 = __shfl_sync(0xffffffffu, v, src);
+      const uint32_t id1 = __shfl_sync(0xffffffffu, id, src);
+      if (mine) {
+        w.minT = t1;
+        w.bu = u1;
+        w.bv = v1;
+        w.best = id1;
+        w.rescale(S);
+        from = ((uint32_t)src & 7u) + 1u;
+        if (w.any) {
+          w.gB = 0u;
+          w.sp = 0;
+          cand = false;
+          from = 8u;
+        }
+      }
+    }
+  }
+}
+
 // The reference's answer for a ray whose walk may have run out of pops, by a
 // block.  The binary tree is searched level by level without the closest hit
 // (its limit only ever rejects more): the accepted inner nodes are kept with
@@ -310,9 +424,11 @@ struct OrdWalk {
 // popped before or at leaf at_k exactly when its own E > at_k.  With at most
 // 2048 pops the last change stands, otherwise the last one whose leaf was
 // among the first 2048, found by halving.  About 25 dependent rounds (the
-// tree's depth) in place of up to 2048; a search that overflows its lists
-// takes the reference's walk instead.
-constexpr uint32_t kCapThreads = 512, kCapFront = 2048, kCapNodes = 6144, kCapHits = 512;
+// tree's depth) in place of up to 2048: 20 us of search and 8 of ordering and
+// counting for a hall ray of 540-1410 accepted nodes and 30-70 hits, the lists
+// sized so that four blocks share an SM.  A search that overflows them takes
+// the reference's walk instead.
+constexpr uint32_t kCapThreads = 256, kCapFront = 1024, kCapNodes = 2048, kCapHits = 192;
 struct CapShared {
   uint2 front[2][kCapFront];  // {node, end of its subtree}
   float near[kCapNodes];
@@ -320,7 +436,7 @@ struct CapShared {
   float4 hit[kCapHits];                     // t, triangle, u, v
   float hitNear[kCapHits], dist[kCapHits];
   uint32_t hitLeaf[kCapHits], order[kCapHits], at[kCapHits], what[kCapHits];
-  uint32_t frontN[3], nodeN, hitN, over, changes, sum[kCapThreads / 32];
+  uint32_t frontN[3], nodeN, hitN, over, changes, sum[32];
   float4 answer;
   uint32_t found;
 };
@@ -331,7 +447,7 @@ __device__ __forceinline__ uint32_t cap_sum(CapShared& c, uint32_t v) {
   if ((threadIdx.x & 31u) == 0u) c.sum[threadIdx.x >> 5] = v;
   __syncthreads();
   uint32_t t = 0;
-  for (uint32_t k = 0; k < kCapThreads / 32; k++) t += c.sum[k];
+  for (uint32_t k = 0; k < blockDim.x / 32; k++) t += c.sum[k];
   return t;
 }
 
@@ -340,7 +456,7 @@ __device__ __forceinline__ uint32_t cap_sum(CapShared& c, uint32_t v) {
 __device__ __forceinline__ void resolve_capped(const DevScene& S, CapShared& c, gb::f3 o, gb::f3 d, float maxDist,
                                                float eps, bool any) {
   using namespace gb;
-  const uint32_t tid = threadIdx.x;
+  const uint32_t tid = threadIdx.x, stride = blockDim.x;
   const f3 inv = mk(rcp_(escape_zero(d.x)), rcp_(escape_zero(d.y)), rcp_(escape_zero(d.z)));
   const f3 oe = o + eps * d;
   __syncthreads();
@@ -359,7 +475,7 @@ __device__ __forceinline__ void resolve_capped(const DevScene& S, CapShared& c, 
     if (n == 0u) break;  // (an overflow ends by itself: nothing more is pushed)
     uint32_t* nextN = &c.frontN[(level + 1u) % 3u];
     if (tid == 0) c.frontN[(level + 2u) % 3u] = 0u;
-    for (uint32_t i = tid; i < n; i += kCapThreads) {
+    for (uint32_t i = tid; i < n; i += stride) {
       const uint2 e = c.front[cur][i];
       const uint32_t id = e.x, E = e.y;
       float4 a, b;
@@ -430,7 +546,7 @@ __device__ __forceinline__ void resolve_capped(const DevScene& S, CapShared& c, 
   // the hits in the reference's order: leaves from the largest node id down,
   // inside a leaf by triangle
   const uint32_t nh = c.hitN;
-  for (uint32_t i = tid; i < nh; i += kCapThreads) {
+  for (uint32_t i = tid; i < nh; i += stride) {
     const uint32_t leaf = c.hitLeaf[i], t = __float_as_uint(c.hit[i].y);
     uint32_t rank = 0;
     for (uint32_t j = 0; j < nh; j++)
@@ -475,7 +591,7 @@ __device__ __forceinline__ void resolve_capped(const DevScene& S, CapShared& c, 
   // pops of nodes whose subtree ends after `upto`
   auto pops = [&](uint32_t upto) {
     uint32_t v = tid == 0 ? 1u : 0u;  // the root
-    for (uint32_t i = tid; i < c.nodeN; i += kCapThreads) {
+    for (uint32_t i = tid; i < c.nodeN; i += stride) {
       const uint32_t E = c.end[i];
       uint32_t lo = 0, hi = any ? 0u : n;  // changes with at >= E
       while (lo < hi) {
