@@ -302,7 +302,8 @@ struct gbpt_renderer {
   bool alloc = false;
   RenderBuffers rb{};
   AdaptBuffers ab{};
-  float *result = nullptr, *gpos = nullptr, *gnorm = nullptr, *gdiff = nullptr, *gauss = nullptr;
+  float *result = nullptr, *gpos = nullptr, *gnorm = nullptr, *gdiff = nullptr;
+  float gauss[64] = {0};  // the filter's spatial weights
   // filter-only mode: first-hit emissive, direct-light and 1 - potential means,
   // the second ping-pong filter plane and the "Prob" view scratch plane
   float *gemis = nullptr, *direct = nullptr, *pot = nullptr, *filtered2 = nullptr, *probView = nullptr;
@@ -402,7 +403,6 @@ struct gbpt_renderer {
     dfree(ab.pred);
     dfree(ab.tileErr);
     bilatOut = nullptr;
-    dfree(gauss);
     dfree(sampleN);
     if (hostResult) cudaFreeHost(hostResult);
     hostResult = nullptr;
@@ -580,7 +580,6 @@ gbpt_status ensure_alloc(gbpt_renderer* r) {
   CK(cudaMemsetAsync(r->rb.m2, 0, np * 12, r->st));
   CK(cudaMemsetAsync(r->rb.hist, 0, nTiles * 32, r->st));
   CK(dalloc(&r->sampleN, np));
-  CK(dalloc(&r->gauss, 64));
   CK(dalloc(&r->ab.err, np));
   CK(dalloc(&r->ab.cnt, np));
   CK(dalloc(&r->ab.off, np));
@@ -641,15 +640,12 @@ cudaEvent_t mark(gbpt_renderer* r, int phase, bool timing) {
   return e;
 }
 
-gbpt_status ensure_gauss(gbpt_renderer* r, float delta, uint32_t radius, cudaStream_t st) {
+void ensure_gauss(gbpt_renderer* r, float delta, uint32_t radius) {
   if (r->gaussKey[0] != delta || r->gaussKey[1] != (float)radius) {
-    float g[64] = {0};
-    gaussian_table_host(delta, radius, g);
-    CK(cudaMemcpyAsync(r->gauss, g, sizeof(g), cudaMemcpyHostToDevice, st));
+    gaussian_table_host(delta, radius, r->gauss);
     r->gaussKey[0] = delta;
     r->gaussKey[1] = (float)radius;
   }
-  return GBPT_OK;
 }
 
 // Filter stage of the filter-only mode (src/cudaRTBDPTStreamBilat.cu:1418-1432):
@@ -660,8 +656,7 @@ gbpt_status ensure_gauss(gbpt_renderer* r, float delta, uint32_t radius, cudaStr
 gbpt_status bilat_filter(gbpt_renderer* r, cudaStream_t st, bool timing) {
   const gbpt_params& p = r->p;
   const float delta = p.filter_sigma_spatial > 0.f ? p.filter_sigma_spatial : p.bilat_color_eud;
-  gbpt_status e = ensure_gauss(r, delta, p.bilat_radius, st);
-  if (e != GBPT_OK) return e;
+  ensure_gauss(r, delta, p.bilat_radius);
   const float* src = r->result;
   const int dm = (int)r->debugMode;
   if (dm == 2 || dm == 3) {
@@ -813,8 +808,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
     const bool budgeted = adaptive && r->frame >= r->p.warmup_frames;
     if (budgeted) {
       float delta = r->p.filter_sigma_spatial > 0.f ? r->p.filter_sigma_spatial : r->p.filter_color_eud;
-      gbpt_status ge = ensure_gauss(r, delta, r->p.filter_radius, st);
-      if (ge != GBPT_OK) return ge;
+      ensure_gauss(r, delta, r->p.filter_radius);
       CK(launch_bilateral(r->result, r->gpos, r->gnorm, r->p.filter_diffuse ? r->gdiff : nullptr, r->W, r->H,
                           r->p.filter_color_eud, r->p.filter_pos_eud, r->p.filter_norm_eud, r->p.filter_diff_eud,
                           r->p.filter_radius, r->gauss, r->ab.filtered, st));
@@ -1640,8 +1634,7 @@ gbpt_status gbpt_renderer_features(gbpt_renderer* r, float* out, uint32_t capaci
   a.moments = 1;
   for (int k = 0; k < 3; k++) a.camPos[k] = r->camBasis[k];
   const float delta = r->p.filter_sigma_spatial > 0.f ? r->p.filter_sigma_spatial : r->p.filter_color_eud;
-  gbpt_status ge = ensure_gauss(r, delta, r->p.filter_radius, st);
-  if (ge != GBPT_OK) return ge;
+  ensure_gauss(r, delta, r->p.filter_radius);
   CK(launch_bilateral(r->result, r->gpos, r->gnorm, r->p.filter_diffuse ? r->gdiff : nullptr, r->W, r->H,
                       r->p.filter_color_eud, r->p.filter_pos_eud, r->p.filter_norm_eud, r->p.filter_diff_eud,
                       r->p.filter_radius, r->gauss, r->ab.filtered, st));
@@ -1903,13 +1896,10 @@ gbpt_status gbpt_bilateral(const float* color, const float* pos, const float* no
   if (!color || !pos || !norm || !g || !out) return fail(GBPT_ERR_INVALID_ARG, "NULL argument");
   if (radius > 31 || width == 0 || height == 0) return fail(GBPT_ERR_INVALID_ARG, "bad size or radius");
   const size_t n = (size_t)width * height * 3;
-  float* dg = nullptr;
-  CK(dalloc(&dg, 2 * radius + 1));
-  CK(cudaMemcpy(dg, g, (2 * radius + 1) * 4, cudaMemcpyHostToDevice));
   gbpt_status st = GBPT_OK;
   if (is_device) {
     cudaError_t e = launch_bilateral(color, pos, norm, emit, width, height, color_eud, pos_eud, norm_eud, emit_eud,
-                                     radius, dg, out, nullptr);
+                                     radius, g, out, nullptr);
     if (!e) e = cudaDeviceSynchronize();
     if (e) st = fail(GBPT_ERR_CUDA, std::string("bilateral: ") + cudaGetErrorString(e));
   } else {
@@ -1922,13 +1912,12 @@ gbpt_status gbpt_bilateral(const float* color, const float* pos, const float* no
       if (!e && k < 4) e = cudaMemcpy(d[k], src[k], n * 4, cudaMemcpyHostToDevice);
     }
     if (!e)
-      e = launch_bilateral(d[0], d[1], d[2], d[3], width, height, color_eud, pos_eud, norm_eud, emit_eud, radius, dg,
+      e = launch_bilateral(d[0], d[1], d[2], d[3], width, height, color_eud, pos_eud, norm_eud, emit_eud, radius, g,
                            d[4], nullptr);
     if (!e) e = cudaMemcpy(out, d[4], n * 4, cudaMemcpyDeviceToHost);
     for (int k = 0; k < 5; k++) dfree(d[k]);
     if (e) st = fail(GBPT_ERR_CUDA, std::string("bilateral: ") + cudaGetErrorString(e));
   }
-  dfree(dg);
   return st;
 }
 

@@ -12,7 +12,10 @@
 //               instead of float atomics, so the result does not depend on timing.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <type_traits>
 
 #include <cstddef>
 
@@ -65,11 +68,40 @@ __device__ __forceinline__ float exp_nonpos_p(float x) {
   return (x < -87.0f) ? 0.0f : res;
 }
 
+// How the tile kernel takes a plane's -mod / c2, fixed at compile time (branches
+// on it inside the tap cost a quarter of a pass): c2 from bilateral_c2, ny = -1/c2
+// correctly rounded.
+//   kQuoMul    c2 < 0: a product (neg_ratio)
+//   kQuoOnce, kQuoTwice  Markstein's quotient: the product with the reciprocal,
+//              corrected by exact multiply-add residuals to the correctly rounded
+//              quotient -- one correction of a value within one unit of the last
+//              place, which the product is when the reciprocal's relative error is
+//              at most 2^-25, else a second (checked against the division over every
+//              mantissa for 320 divisors).  Quotients past 128 are all zero weights:
+//              mod is held there, so infinities stay out of the residuals (a NaN
+//              passes); a quotient too small for exact residuals is one whose
+//              exponential is 1 whatever its last bits.  c2 in [2^-40, 2^40].
+//   kQuoDiv    the division
+enum BilatQuo : int { kQuoMul = 0, kQuoOnce = 1, kQuoTwice = 2, kQuoDiv = 3 };
+struct BilatDiv {
+  float c2, ny;
+};
+template <int kQuo>
+__device__ __forceinline__ float neg_quotient(float mod, BilatDiv v) {
+  if constexpr (kQuo == kQuoMul) return mod * v.c2;
+  if constexpr (kQuo == kQuoDiv) return neg_ratio(mod, v.c2);
+  const float m = mod > 128.f * v.c2 ? 128.f * v.c2 : mod;
+  const float q0 = m * v.ny;
+  const float q1 = gb::fma_(gb::fma_(q0, v.c2, m), v.ny, q0);
+  return kQuo == kQuoOnce ? q1 : gb::fma_(gb::fma_(q1, v.c2, m), v.ny, q1);
+}
+
 // eucl() for the tile kernel: -mod / c2 <= 0 (or NaN) for c2 >= 0
-__device__ __forceinline__ float eucl_nonpos(float ax, float ay, float az, float bx, float by, float bz, float c2) {
+template <int kQuo>
+__device__ __forceinline__ float eucl_nonpos(float ax, float ay, float az, float bx, float by, float bz, BilatDiv v) {
   float dx = bx - ax, dy = by - ay, dz = bz - az;
   float mod = (dx * dx + dy * dy) + dz * dz;
-  return exp_nonpos_p(neg_ratio(mod, c2));
+  return exp_nonpos_p(neg_quotient<kQuo>(mod, v));
 }
 
 // Tap (x+j, y+i) with the reference's unsigned arithmetic: a coordinate left
@@ -83,13 +115,14 @@ __device__ __forceinline__ uint32_t wrapc(int g, uint32_t n) { return ((uint32_t
 // records start 12 words apart and cover all 32 banks once: no conflicts.
 // kR > 0 fixes the radius at compile time (the tap row is unrolled and its
 // weights live in registers); kR == 0 takes r at run time.
-template <bool kEmit, int kR>
+// kColor, kOther: how the colour plane's and the other planes' quotients are taken.
+template <bool kEmit, int kR, int kColor, int kOther>
 __global__ void __launch_bounds__(kTile* kTile) k_bilateral_tile(const float* __restrict__ color,
                                                                   const float* __restrict__ pos,
                                                                   const float* __restrict__ norm,
                                                                   const float* __restrict__ emit, uint32_t W,
-                                                                  uint32_t H, float cc2, float pc2, float nc2,
-                                                                  float ec2, int rArg, const float* __restrict__ g,
+                                                                  uint32_t H, BilatDiv cc2, BilatDiv pc2,
+                                                                  BilatDiv nc2, BilatDiv ec2, int rArg, BilatTable g,
                                                                   float* __restrict__ out) {
   extern __shared__ float4 smv[];
   const int r = kR > 0 ? kR : rArg;
@@ -98,7 +131,7 @@ __global__ void __launch_bounds__(kTile* kTile) k_bilateral_tile(const float* __
   float4* tile = smv + (2 * r + 1 + 3) / 4;
   const int x0 = blockIdx.x * kTile - r, y0 = blockIdx.y * kTile - r;
   const int tid = threadIdx.y * kTile + threadIdx.x;
-  for (int k = tid; k < 2 * r + 1; k += kTile * kTile) sg[k] = g[k];
+  for (int k = tid; k < 2 * r + 1; k += kTile * kTile) sg[k] = g.w[k];
   for (int k = tid; k < T * T; k += kTile * kTile) {
     int ty = k / T, tx = k - ty * T;
     uint32_t gx = wrapc(x0 + tx, W), gy = wrapc(y0 + ty, H);
@@ -118,10 +151,10 @@ __global__ void __launch_bounds__(kTile* kTile) k_bilateral_tile(const float* __
   // one tap, in the reference's order of products and sums
   auto tap = [&](const float4* q, float f) {
     const float4 A = q[0], B = q[1], C = q[2];
-    f = f * eucl_nonpos(A.x, A.y, A.z, cA.x, cA.y, cA.z, cc2);
-    f = f * eucl_nonpos(A.w, B.x, B.y, cA.w, cB.x, cB.y, pc2);
-    f = f * eucl_nonpos(B.z, B.w, C.x, cB.z, cB.w, cC.x, nc2);
-    if (kEmit) f = f * eucl_nonpos(C.y, C.z, C.w, cC.y, cC.z, cC.w, ec2);
+    f = f * eucl_nonpos<kColor>(A.x, A.y, A.z, cA.x, cA.y, cA.z, cc2);
+    f = f * eucl_nonpos<kOther>(A.w, B.x, B.y, cA.w, cB.x, cB.y, pc2);
+    f = f * eucl_nonpos<kOther>(B.z, B.w, C.x, cB.z, cB.w, cC.x, nc2);
+    if (kEmit) f = f * eucl_nonpos<kOther>(C.y, C.z, C.w, cC.y, cC.z, cC.w, ec2);
     tx = tx + f * A.x;
     ty = ty + f * A.y;
     tz = tz + f * A.z;
@@ -142,6 +175,7 @@ __global__ void __launch_bounds__(kTile* kTile) k_bilateral_tile(const float* __
     for (int i = 0; i <= 2 * r; i++) {
       const float gi = sg[i];
       const float4* row = tile + 3 * (size_t)((threadIdx.y + i) * T + threadIdx.x);
+#pragma unroll 4
       for (int j = 0; j <= 2 * r; j++) tap(row + 3 * j, gi * sg[j]);
     }
   }
@@ -156,7 +190,7 @@ template <bool kEmit>
 __global__ void k_bilateral_direct(const float* __restrict__ color, const float* __restrict__ pos,
                                    const float* __restrict__ norm, const float* __restrict__ emit, uint32_t W,
                                    uint32_t H, float cc2, float pc2, float nc2, float ec2, int r,
-                                   const float* __restrict__ g, float* __restrict__ out) {
+                                   BilatTable g, float* __restrict__ out) {
   const uint32_t x = blockIdx.x * kTile + threadIdx.x, y = blockIdx.y * kTile + threadIdx.y;
   if (x >= W || y >= H) return;
   const size_t c = 3 * ((size_t)y * W + x);
@@ -164,7 +198,7 @@ __global__ void k_bilateral_direct(const float* __restrict__ color, const float*
   for (int i = -r; i <= r; i++)
     for (int j = -r; j <= r; j++) {
       size_t q = 3 * ((size_t)wrapc((int)y + i, H) * W + wrapc((int)x + j, W));
-      float f = g[i + r] * g[j + r];
+      float f = g.w[i + r] * g.w[j + r];
       f = f * eucl(color[q], color[q + 1], color[q + 2], color[c], color[c + 1], color[c + 2], cc2);
       f = f * eucl(pos[q], pos[q + 1], pos[q + 2], pos[c], pos[c + 1], pos[c + 2], pc2);
       f = f * eucl(norm[q], norm[q + 1], norm[q + 2], norm[c], norm[c + 1], norm[c + 2], nc2);
@@ -911,28 +945,53 @@ float bilateral_c2(float d) {
   return c2;
 }
 
+// Hall 1280x720, radius 4, three planes, colour delta 50 (c2 = 5000): 0.300 -> 0.200
+// ms per pass against the division; radius 9, four planes, 1003x617: 1.12 -> 0.82.
+static BilatDiv bilateral_div(float c2) { return BilatDiv{c2, c2 > 0.f ? -(1.f / c2) : 0.f}; }
+static int bilateral_quo(float c2) {
+  if (c2 < 0.f) return kQuoMul;
+  if (!(c2 >= 0x1p-40f && c2 <= 0x1p40f)) return kQuoDiv;
+  return std::fabs((double)(1.f / c2) * (double)c2 - 1.0) <= 0x1p-25 ? kQuoOnce : kQuoTwice;  // exact in double
+}
+
 cudaError_t launch_bilateral(const float* color, const float* pos, const float* norm, const float* emit, uint32_t W,
                              uint32_t H, float ceud, float peud, float neud, float eeud, uint32_t radius,
-                             const float* g, float* out, cudaStream_t st) {
+                             const float* weights, float* out, cudaStream_t st) {
   const float cc2 = bilateral_c2(ceud), pc2 = bilateral_c2(peud), nc2 = bilateral_c2(neud), ec2 = bilateral_c2(eeud);
   dim3 grid((W + kTile - 1) / kTile, (H + kTile - 1) / kTile), block(kTile, kTile);
   const int r = (int)radius;
   const int T = kTile + 2 * r;
+  BilatTable g{};
+  std::memcpy(g.w, weights, (2 * r + 1) * sizeof(float));
   const size_t smem = ((size_t)(2 * r + 1 + 3) / 4 + 3 * (size_t)T * T) * sizeof(float4);
   if (smem <= 200 * 1024) {
-    auto tile = [&](auto kern) {
+    // the cases worth a kernel of their own: products throughout, products but for
+    // the colour plane (the adaptive modes' defaults), quotients throughout (a
+    // product is the quotient by the same c2 as well); else the division
+    const int qc = bilateral_quo(cc2);
+    int qo = std::max(bilateral_quo(pc2), bilateral_quo(nc2));
+    if (emit) qo = std::max(qo, bilateral_quo(ec2));
+    auto tile = [&](auto kern, auto div) {
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      kern<<<grid, block, smem, st>>>(color, pos, norm, emit, W, H, cc2, pc2, nc2, ec2, r, g, out);
+      kern<<<grid, block, smem, st>>>(color, pos, norm, emit, W, H, div(cc2), div(pc2), div(nc2), div(ec2), r, g, out);
     };
-    if (emit) {
-      if (r == 4) tile(k_bilateral_tile<true, 4>);
-      else if (r == 5) tile(k_bilateral_tile<true, 5>);
-      else tile(k_bilateral_tile<true, 0>);
-    } else {
-      if (r == 4) tile(k_bilateral_tile<false, 4>);
-      else if (r == 5) tile(k_bilateral_tile<false, 5>);
-      else tile(k_bilateral_tile<false, 0>);
-    }
+    auto pick = [&](auto e, auto rr) {
+      constexpr bool kE = decltype(e)::value;
+      constexpr int kRr = decltype(rr)::value;
+      const auto quo = [](float c2) { return bilateral_div(c2 < 0.f ? -1.f / c2 : c2); };
+      if (qo == kQuoMul && qc == kQuoMul) tile(k_bilateral_tile<kE, kRr, kQuoMul, kQuoMul>, bilateral_div);
+      else if (qo == kQuoMul && qc == kQuoOnce) tile(k_bilateral_tile<kE, kRr, kQuoOnce, kQuoMul>, bilateral_div);
+      else if (qo == kQuoDiv || qc == kQuoDiv) tile(k_bilateral_tile<kE, kRr, kQuoDiv, kQuoDiv>, bilateral_div);
+      else tile(k_bilateral_tile<kE, kRr, kQuoTwice, kQuoTwice>, quo);
+    };
+    using std::integral_constant;
+    auto by_radius = [&](auto e) {
+      if (r == 4) pick(e, integral_constant<int, 4>());
+      else if (r == 5) pick(e, integral_constant<int, 5>());
+      else pick(e, integral_constant<int, 0>());
+    };
+    if (emit) by_radius(std::true_type());
+    else by_radius(std::false_type());
   } else if (emit) {
     k_bilateral_direct<true><<<grid, block, 0, st>>>(color, pos, norm, emit, W, H, cc2, pc2, nc2, ec2, r, g, out);
   } else {

@@ -245,9 +245,14 @@ struct AdaptBuffers {
 constexpr uint32_t kFeatures = 24;
 constexpr uint32_t kErrMlpTimeout = 256u;  // DevCounters::errFlags bit: an MLP tensor-core wait ran out
 constexpr uint32_t kCoopWords = 8192;  // coop buffer size (uint32 words)
+// spatial weights of a filter, handed to its kernels by value
+struct BilatTable {
+  float w[64];
+};
+// weights: 2 * radius + 1 floats in host memory
 cudaError_t launch_bilateral(const float* color, const float* pos, const float* norm, const float* emit, uint32_t W,
                              uint32_t H, float ceud, float peud, float neud, float eeud, uint32_t radius,
-                             const float* g, float* out, cudaStream_t st);
+                             const float* weights, float* out, cudaStream_t st);
 cudaError_t launch_adapt_budget(const FrameArgs& a, const RenderBuffers& b, const AdaptBuffers& ab,
                                 const float* result, const uint32_t* sampleN, uint32_t desired, cudaStream_t st);
 // the two halves of launch_adapt_budget: per-pixel error (+ partial sums), then
