@@ -14,9 +14,11 @@
 //   * every mbarrier wait is bounded (1 s on %globaltimer): on expiry the
 //     kernel sets an error bit, waits once more (bounded) for its own MMAs,
 //     frees its TMEM and returns.
-// One CTA of 128 threads owns 128 rows (samples); thread r owns row r in
-// every epilogue.  Training: forward, loss, backward through both layers and
-// the weight gradients as tensor-core products over the CTA's rows
+// One CTA of 512 threads owns 128 rows (samples): four warps share 32 rows
+// (a warp reads only the TMEM lanes 32 (w mod 4) ..+31) and take 16 of the 64
+// columns each in every epilogue.  Training: forward, loss, backward through
+// both layers and the weight gradients as tensor-core products over the CTA's
+// rows
 // (dW2 = dZ2^T H1, dW1 = dZ1^T X, with the 64 output rows padded to M = 128
 // by zero rows), accumulated across CTAs with FP32 atomics; then Adam.
 // Rounding points (matched by the CPU oracle): X, W1, W2, w3, H1, dZ2, dZ1
@@ -36,7 +38,7 @@
 namespace gbpt {
 namespace mlp {
 
-constexpr int kIn = 24, kInPad = 32, kHid = 64, kRows = 128, kThreads = 128;
+constexpr int kIn = 24, kHid = 64, kRows = 128, kThreads = 512;
 constexpr int oW1 = 0, oB1 = kHid * kIn, oW2 = oB1 + kHid, oB2 = oW2 + kHid * kHid, oW3 = oB2 + kHid,
               oB3 = oW3 + kHid, kParams = oB3 + 1;  // 5825
 static_assert(kParams == 5825, "parameter layout");
@@ -69,6 +71,7 @@ constexpr uint32_t kInferSmem = sBw2 + tile_bytes(64, 64) + kVecFloats * 4 + 64;
 // the inference kernel requests this much so that at most 4 CTAs (4 x 128
 // TMEM columns = the SM's 512) are resident per SM: tcgen05.alloc never waits
 constexpr uint32_t kInferSmemLaunch = 56 * 1024;
+static_assert(128 * 65 * 4 <= sBw2 + tile_bytes(64, 64), "H2 fits over the operand tiles");
 static_assert(kInferSmem <= kInferSmemLaunch, "inference tile fits");
 static_assert(kTrainSmem <= 200 * 1024, "training tile fits in shared memory");
 
@@ -110,6 +113,7 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t phase) {
 
 // bounded wait for the mbarrier phase; false after ~1 s
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase) {
+  if (mbar_try(bar, phase)) return true;
   const uint64_t t0 = now_ns();
   while (!mbar_try(bar, phase)) {
     if (now_ns() - t0 > 1000000000ull) return false;
@@ -157,8 +161,46 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void st_bf16(uint8_t* base, uint32_t off, float x) {
-  *reinterpret_cast<__nv_bfloat16*>(base + off) = __float2bfloat16_rn(x);
+// eight consecutive columns of a tile row: one 16-byte row of a core matrix
+__device__ __forceinline__ void st_row8(uint8_t* p, const float* v) {
+  uint32_t r[4];
+  for (int i = 0; i < 4; i++) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    r[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  *reinterpret_cast<uint4*>(p) = make_uint4(r[0], r[1], r[2], r[3]);
+}
+
+// eight floats of global memory, by 16-byte loads where the caller's rows allow it
+__device__ __forceinline__ void ld8(const float* __restrict__ p, bool vec, float* v) {
+  if (vec) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+  } else {
+    for (int i = 0; i < 8; i++) v[i] = p[i];
+  }
+}
+
+// Four 8 x 8 core matrices transposed: lane l names row l & 7 of matrix l >> 3
+// in the source and in the destination.  The element-wise 2-byte stores of the
+// transposed tiles were four-way bank conflicts, 64 to 128 a thread.
+__device__ __forceinline__ void transpose4(uint32_t src, uint32_t dst) {
+  uint32_t r0, r1, r2, r3;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+               : "r"(src)
+               : "memory");
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(r0), "r"(r1), "r"(r2),
+               "r"(r3)
+               : "memory");
+}
+
+// this warp's 32 rows x 16 columns of a 128 x 64 tile, into its 64 x 128 transpose
+__device__ __forceinline__ void transpose_block(uint32_t tile, uint32_t tileT, uint32_t rowCore, uint32_t colCore) {
+  const uint32_t lane = threadIdx.x & 31u, a = lane >> 3, j = (lane & 7u) * 16u;
+  __syncwarp();
+  for (uint32_t c = colCore; c < colCore + 2; c++)
+    transpose4(tile + (rowCore + a) * (64u * 16u) + c * 128u + j, tileT + c * (128u * 16u) + (rowCore + a) * 128u + j);
 }
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -166,9 +208,31 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-__device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float z) {
-  return 0.5f * (1.f + erff(z * 0.70710678118654752f)) + z * expf(-0.5f * z * z) * 0.39894228040143268f;
+// Sums of 16 columns over the warp's 32 rows: halves of the columns are handed
+// over while halves of the rows are added, 31 shuffles in place of 80, and every
+// lane ends with the sum of column lane >> 1 (the additions of warp_sum's tree).
+__device__ __forceinline__ float col_sums16(const float* in) {
+  const uint32_t lane = threadIdx.x & 31u;
+  float v[16];
+#pragma unroll
+  for (int i = 0; i < 16; i++) v[i] = in[i];
+#pragma unroll
+  for (int h = 8; h > 0; h >>= 1) {
+    const bool up = (lane & (uint32_t)(2 * h)) != 0;
+#pragma unroll
+    for (int i = 0; i < h; i++) {
+      const float give = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// GELU and its derivative from e = erf(z / sqrt 2), which both need
+__device__ __forceinline__ float gelu_erf(float z) { return erff(z * 0.70710678118654752f); }
+__device__ __forceinline__ float gelu(float z, float e) { return 0.5f * z * (1.f + e); }
+__device__ __forceinline__ float gelu_grad(float z, float e) {
+  return 0.5f * (1.f + e) + z * expf(-0.5f * z * z) * 0.39894228040143268f;
 }
 
 // TMEM allocation by warp 0; returns the base address through the smem slot
@@ -181,24 +245,49 @@ __device__ __forceinline__ void tmem_free(uint32_t base, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
 }
 
-// Stage the weights of both MMA layers (and their biases, w3) from the FP32 master vector.
+// Stage the weights of both MMA layers (and their biases, w3) from the FP32
+// master vector.  A thread takes eight columns of one row, a warp eight rows,
+// so that each store is a 16-byte row of a core matrix without bank conflicts.
 __device__ void stage_weights(uint8_t* sm, const float* __restrict__ theta, bool transposeW2) {
-  const uint32_t t = threadIdx.x;
-  for (uint32_t e = t; e < 64u * 32u; e += kThreads) {  // W1 (64 x 32, K 24..31 zero)
-    const uint32_t o = e >> 5, k = e & 31u;
-    st_bf16(sm + sBw1, kmaj(o, k, 32), k < (uint32_t)kIn ? theta[oW1 + o * kIn + k] : 0.f);
+  const uint32_t t = threadIdx.x, a = (t >> 3) & 3u, j = t & 7u;
+  float v[8];
+  if (t < 256) {  // W1 (64 x 32, K 24..31 zero)
+    const uint32_t o = (t >> 5) * 8u + j;
+    for (int i = 0; i < 8; i++) v[i] = 0.f;
+    if (a < 3) ld8(theta + oW1 + o * kIn + a * 8u, true, v);
+    st_row8(sm + sBw1 + kmaj(o, a * 8u, 32), v);
   }
-  for (uint32_t e = t; e < 64u * 64u; e += kThreads) {  // W2 (o, i) and W2^T (i, o)
-    const uint32_t o = e >> 6, i = e & 63u;
-    const float w = theta[oW2 + e];
-    st_bf16(sm + sBw2, kmaj(o, i, 64), w);
-    if (transposeW2) st_bf16(sm + sBw2t, kmaj(i, o, 64), w);
+  {  // W2 (o, i) and W2^T (i, o): a warp holds four core matrices
+    const uint32_t oc = t >> 6, ic = ((t >> 5) & 1u) * 4u + a;
+    ld8(theta + oW2 + (oc * 8u + j) * kHid + ic * 8u, true, v);
+    st_row8(sm + sBw2 + kmaj(oc * 8u + j, ic * 8u, 64), v);
+    if (transposeW2) {
+      __syncwarp();
+      transpose4(smem_u32(sm + sBw2 + kmaj(oc * 8u + j, ic * 8u, 64)),
+                 smem_u32(sm + sBw2t + kmaj(ic * 8u + j, oc * 8u, 64)));
+    }
   }
   float* vec = reinterpret_cast<float*>(sm + (transposeW2 ? sVec : kInferSmem - kVecFloats * 4 - 64));
   if (t < 64) {
     vec[t] = theta[oB1 + t];
     vec[64 + t] = theta[oB2 + t];
     vec[128 + t] = __bfloat162float(__float2bfloat16_rn(theta[oW3 + t]));
+  }
+}
+
+// Stage the CTA's rows of X (zero past row n and past column 23), and X^T: a
+// warp holds eight rows, a lane eight columns of one.
+__device__ void stage_x(uint8_t* sm, const float* __restrict__ x, uint32_t n, bool transpose) {
+  const uint32_t t = threadIdx.x, a = (t >> 3) & 3u, r = (t >> 5) * 8u + (t & 7u);
+  const uint32_t row = blockIdx.x * kRows + r;
+  const bool vec = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;  // a row is 96 bytes
+  float v[8];
+  for (int i = 0; i < 8; i++) v[i] = 0.f;
+  if (row < n && a < 3) ld8(x + (size_t)row * kIn + a * 8u, vec, v);
+  st_row8(sm + sAx + kmaj(r, a * 8u, 32), v);
+  if (transpose) {
+    __syncwarp();
+    transpose4(smem_u32(sm + sAx + kmaj(r, a * 8u, 32)), smem_u32(sm + sBxt + kmaj(a * 8u + (t & 7u), r & ~7u, 128)));
   }
 }
 
@@ -209,12 +298,19 @@ using namespace mlp;
 
 // ---------------------------------------------------------------------------
 // Inference: y[r] = MLP(x[r]) for n rows of 24 FP32 features.
-__global__ void __launch_bounds__(kThreads, 1) k_mlp_forward(const float* __restrict__ x, uint32_t n,
+// Bound by the chain staging -> MMA -> GELU -> MMA -> GELU of a CTA (a tile's
+// products are 0.4 us of one SM's tensor rate): with one thread a row the
+// 128 GELUs of a row stood one behind another and each scheduler had one warp.
+// The output sum is taken by one thread a row in column order, as before, from
+// shared memory (stride 65: no bank conflicts), so the result keeps its bits.
+// 14400 rows (113 CTAs): 14 -> 7 us; launch and staging are most of the rest.
+__global__ void __launch_bounds__(kThreads, 2) k_mlp_forward(const float* __restrict__ x, uint32_t n,
                                                             const float* __restrict__ theta, float* __restrict__ y,
                                                             uint32_t* err, uint32_t errBit) {
   extern __shared__ __align__(1024) uint8_t sm[];
   const uint32_t t = threadIdx.x, warp = t >> 5;
-  const uint32_t row = blockIdx.x * kRows + t;
+  const uint32_t r = (warp & 3u) * 32u + (t & 31u), c0 = (warp >> 2) * 16u;  // tile row, first column
+  const uint32_t row = blockIdx.x * kRows + r;
   float* vec = reinterpret_cast<float*>(sm + kInferSmem - kVecFloats * 4 - 64);
   uint32_t* slot = reinterpret_cast<uint32_t*>(sm + kInferSmem - 64);
   const uint32_t bar = smem_u32(sm + kInferSmem - 56);
@@ -224,12 +320,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_forward(const float* __rest
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   stage_weights(sm, theta, false);
-  {  // X tile
-    for (int k = 0; k < kInPad; k++) {
-      const float v = (row < n && k < kIn) ? x[(size_t)row * kIn + k] : 0.f;
-      st_bf16(sm + sAx, kmaj(t, k, 32), v);
-    }
-  }
+  stage_x(sm, x, n, false);
   fence_async_smem();
   tc_before();
   __syncthreads();
@@ -244,13 +335,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_forward(const float* __rest
   ok = __syncthreads_and(mbar_wait(bar, phase) ? 1 : 0) != 0;  // block-uniform
   if (ok) phase ^= 1u;
   tc_after();
-  const uint32_t lane0 = (warp * 32u) << 16;
+  const uint32_t lane0 = ((warp & 3u) * 32u) << 16;
   if (ok) {
-    for (int c = 0; c < 64; c += 16) {
-      float z[16];
-      tmem_ld16(tmem + lane0 + tD1 + c, z);
-      for (int j = 0; j < 16; j++) st_bf16(sm + sAh1, kmaj(t, c + j, 64), gelu(z[j] + vec[c + j]));
+    float z[16];
+    tmem_ld16(tmem + lane0 + tD1 + c0, z);
+    for (int j = 0; j < 16; j++) {
+      z[j] += vec[c0 + j];
+      z[j] = gelu(z[j], gelu_erf(z[j]));
     }
+    st_row8(sm + sAh1 + kmaj(r, c0, 64), z);
+    st_row8(sm + sAh1 + kmaj(r, c0 + 8, 64), z + 8);
     fence_async_smem();
   }
   tc_before();
@@ -266,13 +360,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_forward(const float* __rest
     tc_after();
   }
   if (ok) {
-    float acc = theta[oB3];
-    for (int c = 0; c < 64; c += 16) {
-      float z[16];
-      tmem_ld16(tmem + lane0 + tD2 + c, z);
-      for (int j = 0; j < 16; j++) acc += gelu(z[j] + vec[64 + c + j]) * vec[128 + c + j];
+    float* h = reinterpret_cast<float*>(sm);  // the operand tiles are done with: 128 x 65 floats of H2
+    float z[16];
+    tmem_ld16(tmem + lane0 + tD2 + c0, z);
+    for (int j = 0; j < 16; j++) {
+      z[j] += vec[64 + c0 + j];
+      h[r * 65u + c0 + j] = gelu(z[j], gelu_erf(z[j]));
     }
-    if (row < n) y[row] = acc;
+    __syncthreads();
+    if (warp < 4) {
+      float acc = theta[oB3];
+#pragma unroll 16
+      for (int j = 0; j < 64; j++) acc += h[r * 65u + j] * vec[128 + j];
+      if (row < n) y[row] = acc;
+    }
   } else if (t == 0) {
     atomicOr(err, errBit);
   }
@@ -287,13 +388,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_forward(const float* __rest
 
 // ---------------------------------------------------------------------------
 // Training: loss, and the gradient of the mean squared error over n rows
-// accumulated into grad (FP32, kParams).  lossSum receives sum (y - t)^2.
+// accumulated into grad (FP32, kParams; its rows are 16-byte aligned for the
+// vector atomics).  Bound by the CTA's chain of four products and three
+// epilogues, as the forward pass: erf is taken once per pre-activation and kept
+// for the way back, column sums share their shuffles, transposed tiles are
+// written a core matrix at a time, and dW2 goes out under dW1's product.
+// 4096 rows (32 CTAs): 49 -> 12 us.  lossSum receives sum (y - t)^2.
 __global__ void __launch_bounds__(kThreads, 1) k_mlp_train(const float* __restrict__ x, const float* __restrict__ tgt,
                                                           uint32_t n, const float* __restrict__ theta,
                                                           float* __restrict__ grad, float* lossSum, uint32_t* err) {
   extern __shared__ __align__(1024) uint8_t sm[];
   const uint32_t t = threadIdx.x, warp = t >> 5;
-  const uint32_t row = blockIdx.x * kRows + t;
+  const uint32_t r = (warp & 3u) * 32u + (t & 31u), c0 = (warp >> 2) * 16u;  // tile row, first column
+  const uint32_t row = blockIdx.x * kRows + r;
   const bool valid = row < n;
   float* vec = reinterpret_cast<float*>(sm + sVec);
   float* sdb1 = vec + 192;
@@ -316,21 +423,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train(const float* __restri
     *reinterpret_cast<uint4*>(sm + sAdz2t + kmaj(r, k8, 128)) = make_uint4(0, 0, 0, 0);
     *reinterpret_cast<uint4*>(sm + sAdz1t + kmaj(r, k8, 128)) = make_uint4(0, 0, 0, 0);
   }
-  for (int k = 0; k < kInPad; k++) {  // X tile (row-major) and X^T
-    const float v = (valid && k < kIn) ? x[(size_t)row * kIn + k] : 0.f;
-    st_bf16(sm + sAx, kmaj(t, k, 32), v);
-    st_bf16(sm + sBxt, kmaj(k, t, 128), v);
-  }
+  stage_x(sm, x, n, true);
   const float target = valid ? tgt[row] : 0.f;
   fence_async_smem();
   tc_before();
   __syncthreads();
   tc_after();
   const uint32_t tmem = *slot;
-  const uint32_t lane0 = (warp * 32u) << 16;
+  const uint32_t lane0 = ((warp & 3u) * 32u) << 16;
   uint32_t phase = 0;
   bool ok = true;
 
+  float e1[16];  // erf of layer 1's pre-activations, for the way back
   // ---- layer 1: D1 = X W1^T
   if (t == 0) {
     mma_issue(tmem + tD1, smem_u32(sm + sAx), 32, smem_u32(sm + sBw1), 32, 64, 2);
@@ -340,15 +444,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train(const float* __restri
   if (ok) phase ^= 1u;
   tc_after();
   if (ok) {
-    for (int c = 0; c < 64; c += 16) {
-      float z[16];
-      tmem_ld16(tmem + lane0 + tD1 + c, z);
-      for (int j = 0; j < 16; j++) {
-        const float h = gelu(z[j] + vec[c + j]);
-        st_bf16(sm + sAh1, kmaj(t, c + j, 64), h);
-        st_bf16(sm + sBh1t, kmaj(c + j, t, 128), h);
-      }
+    float z[16];
+    tmem_ld16(tmem + lane0 + tD1 + c0, z);
+    for (int j = 0; j < 16; j++) {
+      z[j] += vec[c0 + j];
+      e1[j] = gelu_erf(z[j]);
+      z[j] = gelu(z[j], e1[j]);
     }
+    st_row8(sm + sAh1 + kmaj(r, c0, 64), z);
+    st_row8(sm + sAh1 + kmaj(r, c0 + 8, 64), z + 8);
+    transpose_block(smem_u32(sm + sAh1), smem_u32(sm + sBh1t), r >> 3 & ~3u, c0 >> 3);
     fence_async_smem();
   }
   tc_before();
@@ -365,31 +470,40 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train(const float* __restri
     tc_after();
   }
   if (ok) {
-    float z2[64];
-    for (int c = 0; c < 64; c += 16) tmem_ld16(tmem + lane0 + tD2 + c, z2 + c);
-    float yv = theta[oB3];
-    for (int j = 0; j < 64; j++) {
-      z2[j] += vec[64 + j];
-      yv += gelu(z2[j]) * vec[128 + j];
+    float z2[16], e2[16];
+    float* part = reinterpret_cast<float*>(sm + sAx);  // X is done with: 4 x 128 partial outputs
+    tmem_ld16(tmem + lane0 + tD2 + c0, z2);
+    float yp = 0.f;
+    for (int j = 0; j < 16; j++) {
+      z2[j] += vec[64 + c0 + j];
+      e2[j] = gelu_erf(z2[j]);
+      yp += gelu(z2[j], e2[j]) * vec[128 + c0 + j];
     }
+    part[(warp >> 2) * kRows + r] = yp;
+    __syncthreads();
+    const float yv = theta[oB3] + ((part[r] + part[kRows + r]) + (part[2 * kRows + r] + part[3 * kRows + r]));
     const float dy = valid ? 2.f * (yv - target) / (float)n : 0.f;
-    // column sums over the CTA's rows: a warp butterfly, then one shared atomic per warp
-    const float l2 = warp_sum(valid ? (yv - target) * (yv - target) : 0.f), sdy = warp_sum(dy);
-    if ((t & 31) == 0) {
-      atomicAdd(&sscal[1], l2);
-      atomicAdd(&sscal[0], sdy);
-    }
-    for (int j = 0; j < 64; j++) {
-      const float g3 = warp_sum(dy * gelu(z2[j]));
-      const float dz = dy * vec[128 + j] * gelu_grad(z2[j]);
-      const float g2 = warp_sum(dz);
+    // column sums over the CTA's rows: a warp butterfly, then one shared atomic a warp and column
+    if (warp < 4) {
+      const float l2 = warp_sum(valid ? (yv - target) * (yv - target) : 0.f), sdy = warp_sum(dy);
       if ((t & 31) == 0) {
-        atomicAdd(&sdw3[j], g3);
-        atomicAdd(&sdb2[j], g2);
+        atomicAdd(&sscal[1], l2);
+        atomicAdd(&sscal[0], sdy);
       }
-      st_bf16(sm + sAdz2, kmaj(t, j, 64), dz);
-      st_bf16(sm + sAdz2t, kmaj(j, t, 128), dz);
     }
+    float g3[16], dz[16];
+    for (int j = 0; j < 16; j++) {
+      g3[j] = dy * gelu(z2[j], e2[j]);
+      dz[j] = dy * vec[128 + c0 + j] * gelu_grad(z2[j], e2[j]);
+    }
+    const float s3 = col_sums16(g3), s2 = col_sums16(dz);
+    if ((t & 1) == 0) {
+      atomicAdd(&sdw3[c0 + ((t & 31u) >> 1)], s3);
+      atomicAdd(&sdb2[c0 + ((t & 31u) >> 1)], s2);
+    }
+    st_row8(sm + sAdz2 + kmaj(r, c0, 64), dz);
+    st_row8(sm + sAdz2 + kmaj(r, c0 + 8, 64), dz + 8);
+    transpose_block(smem_u32(sm + sAdz2), smem_u32(sm + sAdz2t), r >> 3 & ~3u, c0 >> 3);
     fence_async_smem();
   }
   tc_before();
@@ -407,24 +521,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train(const float* __restri
     tc_after();
   }
   if (ok) {
-    for (int c = 0; c < 64; c += 16) {
-      float dh[16], z1[16];
-      tmem_ld16(tmem + lane0 + tD3 + c, dh);
-      tmem_ld16(tmem + lane0 + tD1 + c, z1);
-      for (int j = 0; j < 16; j++) {
-        const float dz = dh[j] * gelu_grad(z1[j] + vec[c + j]);
-        const float g1 = warp_sum(dz);
-        if ((t & 31) == 0) atomicAdd(&sdb1[c + j], g1);
-        st_bf16(sm + sAdz1t, kmaj(c + j, t, 128), dz);
-      }
-    }
-    if (warp < 2) {  // rows 0..63 of D4 = dW2[o = t][i] (warps 2-3 hold the zero padding rows)
-      for (int c = 0; c < 64; c += 16) {
-        float g[16];
-        tmem_ld16(tmem + lane0 + tD4 + c, g);
-        for (int j = 0; j < 16; j++) atomicAdd(&grad[oW2 + t * 64 + c + j], g[j]);
-      }
-    }
+    float dh[16], z1[16];
+    tmem_ld16(tmem + lane0 + tD3 + c0, dh);
+    tmem_ld16(tmem + lane0 + tD1 + c0, z1);
+    for (int j = 0; j < 16; j++) dh[j] *= gelu_grad(z1[j] + vec[c0 + j], e1[j]);
+    const float s1 = col_sums16(dh);
+    if ((t & 1) == 0) atomicAdd(&sdb1[c0 + ((t & 31u) >> 1)], s1);
+    // row-major into dZ2's tile, whose products are complete, then transposed
+    st_row8(sm + sAdz2 + kmaj(r, c0, 64), dh);
+    st_row8(sm + sAdz2 + kmaj(r, c0 + 8, 64), dh + 8);
+    transpose_block(smem_u32(sm + sAdz2), smem_u32(sm + sAdz1t), r >> 3 & ~3u, c0 >> 3);
     fence_async_smem();
   }
   tc_before();
@@ -435,18 +541,26 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train(const float* __restri
     mma_issue(tmem + tD5, smem_u32(sm + sAdz1t), 128, smem_u32(sm + sBxt), 128, 32, 8);
     mma_commit(bar);
   }
+  __syncwarp();
+  if (ok && r < 64) {  // meanwhile rows 0..63 of D4 = dW2[o = r][i] (64..127 are the zero padding rows)
+    float g[16];
+    tmem_ld16(tmem + lane0 + tD4 + c0, g);
+    for (int j = 0; j < 16; j += 4)
+      atomicAdd(reinterpret_cast<float4*>(&grad[oW2 + r * kHid + c0 + j]),
+                make_float4(g[j], g[j + 1], g[j + 2], g[j + 3]));
+  }
   if (ok) {
     ok = __syncthreads_and(mbar_wait(bar, phase) ? 1 : 0) != 0;  // block-uniform
     if (ok) phase ^= 1u;
     tc_after();
   }
-  if (ok && warp < 2) {  // rows 0..63 of D5 = dW1[o = t][i], i < 24
-    for (int c = 0; c < 32; c += 16) {
-      float g[16];
-      tmem_ld16(tmem + lane0 + tD5 + c, g);
-      for (int j = 0; j < 16; j++)
-        if (c + j < kIn) atomicAdd(&grad[oW1 + t * kIn + c + j], g[j]);
-    }
+  if (ok && r < 64 && c0 < 32) {  // rows 0..63 of D5 = dW1[o = r][i], i < 24
+    float g[16];
+    tmem_ld16(tmem + lane0 + tD5 + c0, g);
+    for (int j = 0; j < 16; j += 4)
+      if (c0 + j < kIn)
+        atomicAdd(reinterpret_cast<float4*>(&grad[oW1 + r * kIn + c0 + j]),
+                  make_float4(g[j], g[j + 1], g[j + 2], g[j + 3]));
   }
   if (!ok) {
     if (t == 0) atomicOr(err, kErrTimeout);
