@@ -413,6 +413,56 @@ __device__ __forceinline__ void coop_walk(const DevScene& S, OrdWalk& w, uint2* 
   }
 }
 
+// The walks of a warp's last few lanes (at most four bits of `live`) to their
+// ends, eight lanes each: the k-th live lane's walk and stack are copied to
+// lanes 8k .. 8k + 7 and its result is taken back.  Warp-uniform call.
+__device__ __forceinline__ void gather_walks(const DevScene& S, OrdWalk& w, uint2* stack, uint32_t live) {
+  using namespace gb;
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t m = live;
+  for (uint32_t k = lane >> 3; k > 0; k--) m &= m - 1u;
+  const bool have = m != 0u;
+  const int src = have ? __ffs((int)m) - 1 : (int)lane;
+  const auto from = [src](float x) { return __shfl_sync(0xffffffffu, x, src); };
+  const auto fromU = [src](uint32_t x) { return __shfl_sync(0xffffffffu, x, src); };
+  const int mine = (live >> lane) & 1u ? w.sp : 0;
+  const int deepest = __reduce_max_sync(0xffffffffu, mine);
+  // entry i moves to entry i, read before it is written: no second stack
+  for (int i = 0; i < deepest; i++) {
+    const uint2 e = i < mine ? stack[i] : make_uint2(0u, 0u);
+    stack[i] = make_uint2(fromU(e.x), fromU(e.y));
+  }
+  w.o = mk(from(w.o.x), from(w.o.y), from(w.o.z));
+  w.d = mk(from(w.d.x), from(w.d.y), from(w.d.z));
+  w.inv = mk(from(w.inv.x), from(w.inv.y), from(w.inv.z));
+  w.minT = from(w.minT);
+  w.scale = from(w.scale);
+  w.bu = from(w.bu);
+  w.bv = from(w.bv);
+  w.best = fromU(w.best);
+  w.gA = fromU(w.gA);
+  w.gB = fromU(w.gB);
+  w.bound = fromU(w.bound);
+  w.sp = __shfl_sync(0xffffffffu, mine, src);
+  w.any = __shfl_sync(0xffffffffu, (int)w.any, src) != 0;
+  w.eps = from(w.eps);
+  coop_walk(S, w, stack, have);
+  // the ray goes back too: a walk past the pop bound is run again from it
+  const int home = (int)(8u * (uint32_t)__popc(live & ((1u << lane) - 1u))) & 31;
+  const auto back = [home](float x) { return __shfl_sync(0xffffffffu, x, home); };
+  w.o = mk(back(w.o.x), back(w.o.y), back(w.o.z));
+  w.d = mk(back(w.d.x), back(w.d.y), back(w.d.z));
+  w.minT = back(w.minT);
+  w.bu = back(w.bu);
+  w.bv = back(w.bv);
+  w.best = __shfl_sync(0xffffffffu, w.best, home);
+  w.bound = __shfl_sync(0xffffffffu, w.bound, home);
+  w.any = __shfl_sync(0xffffffffu, (int)w.any, home) != 0;
+  w.eps = back(w.eps);
+  w.gB = 0u;
+  w.sp = 0;
+}
+
 // The reference's answer for a ray whose walk may have run out of pops, by a
 // block.  The binary tree is searched level by level without the closest hit
 // (its limit only ever rejects more): the accepted inner nodes are kept with
