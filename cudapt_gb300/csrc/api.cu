@@ -293,6 +293,18 @@ enum Phase { kPhLight = 0, kPhTrace, kPhShade, kPhShadow, kPhFilter, kPhAdapt, k
 
 }  // namespace
 
+// Frames of one call traced at once (render_impl).  A frame's last bounces
+// leave half of the machine idle: the mean warp of the tail kernel lives half
+// as long as the longest one (Cornell 256x256 262 of 550 thousand cycles,
+// unidirectional 333x217 image 544 of 1074), and the next frame's paths fill
+// that.  Whole images, 1 / 2 / 3 / 4 frames at once (ms): Cornell 256x256 3.59 /
+// 2.66 / 2.48 / 2.60, unidirectional 333x217 4.15 / 3.04 / 2.91 / 2.89, binary
+// allocator 500x375 9.48 / 8.25 / 7.77 / 7.62, filtered 641x359 6.35 / 5.24 /
+// 5.27 / 4.85, adaptive hall 1280x720 33.4 / 30.7 / 31.1 (its walks fill the
+// machine by themselves): the lines lie between those sizes.
+constexpr uint32_t kFrameSlots = 4;
+uint32_t frame_slots(size_t paths) { return paths < (1u << 17) ? 3u : paths < (1u << 19) ? kFrameSlots : 2u; }
+
 struct gbpt_renderer {
   uint32_t W = 0, H = 0;
   int32_t mode = GBPT_MODE_BDPT_SC;
@@ -336,6 +348,15 @@ struct gbpt_renderer {
   cudaStream_t stBand[kMaxBands] = {};
   cudaEvent_t evFork = nullptr, evJoin[kMaxBands] = {};
   uint32_t lastBands = 1;
+  // frames in flight: the buffers, stream and last event of the frames traced
+  // beside the work stream's (slot 0 is rb on the work stream)
+  RenderBuffers slot[kFrameSlots - 1];
+  char* slotMem = nullptr;
+  uint32_t slots = 1;     // rb and those laid out in slotMem
+  uint32_t slotConn = 0;  // connection depth the slots were laid out for
+  cudaStream_t stSlot[kFrameSlots - 1] = {};
+  cudaEvent_t evSlot[kFrameSlots] = {}, evCall = nullptr;
+  uint32_t lastSlot = 0, lastSlots = 1;  // of the last frame; used by the last call
   bool refWalk = false;  // this sequence's lists of walks past the pop bound ran full: node-by-node walk
   // window of a larger image (gbpt_renderer_set_window); the whole image by default
   uint32_t winX0 = 0, winY0 = 0, fullW = 0, fullH = 0;
@@ -356,6 +377,9 @@ struct gbpt_renderer {
   bool lastTraced = true;  // the last frame traced camera paths (filter-only mode may only filter)
 
   void free_dev() {
+    for (cudaStream_t x : stSlot)
+      if (x) cudaStreamSynchronize(x);
+    dfree(slotMem);
     for (int k = 0; k < 2; k++) rb.wave[k] = Wave{};
     dfree(waveMem);
     dfree(rb.hit);
@@ -411,7 +435,14 @@ struct gbpt_renderer {
   }
   ~gbpt_renderer() {
     if (st) cudaStreamSynchronize(st);
+    for (cudaStream_t x : stSlot)
+      if (x) cudaStreamSynchronize(x);
     free_dev();
+    for (cudaStream_t x : stSlot)
+      if (x) cudaStreamDestroy(x);
+    for (cudaEvent_t e : evSlot)
+      if (e) cudaEventDestroy(e);
+    if (evCall) cudaEventDestroy(evCall);
     for (auto e : evPool) cudaEventDestroy(e);
     for (cudaGraphExec_t& x : gexec)
       if (x) cudaGraphExecDestroy(x);
@@ -677,7 +708,21 @@ gbpt_status bilat_filter(gbpt_renderer* r, cudaStream_t st, bool timing) {
   return GBPT_OK;
 }
 
-gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, bool timing) {
+bool adaptive_mode(const gbpt_renderer* r) {
+  return r->mode == GBPT_MODE_BDPT_SC_ADAP_BILAT || r->mode == GBPT_MODE_BDPT_SC_ADAP_BILAT_BINARY;
+}
+// second moments and path-length counts are kept for a learned allocator
+bool keeps_moments(const gbpt_renderer* r) {
+  return (r->mlp != nullptr && r->mode == GBPT_MODE_BDPT_SC_ADAP_BILAT) || (r->collect && adaptive_mode(r));
+}
+
+// Where a frame of a call runs: its slot, and whether the call's frames overlap.
+struct FramePlace {
+  uint32_t slot = 0;
+  bool overlap = false;
+};
+
+gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, bool timing, FramePlace at) {
   float right[3], up[3];
   cam_basis(*cam, right, up);
   float basis9[9] = {cam->pos[0], cam->pos[1], cam->pos[2], cam->dir[0], cam->dir[1],
@@ -724,7 +769,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
   a.lightPaths = r->p.light_paths;
   for (int k = 0; k < 3; k++) a.env[k] = r->p.env[k];
   a.useEnv = (r->p.env[0] != 0.f || r->p.env[1] != 0.f || r->p.env[2] != 0.f) ? 1u : 0u;
-  const bool adaptive = r->mode == GBPT_MODE_BDPT_SC_ADAP_BILAT || r->mode == GBPT_MODE_BDPT_SC_ADAP_BILAT_BINARY;
+  const bool adaptive = adaptive_mode(r);
   const bool binary = r->mode == GBPT_MODE_BDPT_SC_ADAP_BILAT_BINARY;
   if (adaptive && (fullW != r->W || fullH != r->H))
     return fail(GBPT_ERR_STATE, "the adaptive modes render whole images only: their sample budget and filter "
@@ -736,7 +781,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
   a.bilat = bilat ? 1u : 0u;
   // learned allocator (PLL adaptive mode): second moments and path-length counts
   const bool learned = r->mlp != nullptr && r->mode == GBPT_MODE_BDPT_SC_ADAP_BILAT;
-  a.moments = (learned || (r->collect && adaptive)) ? 1u : 0u;
+  a.moments = keeps_moments(r) ? 1u : 0u;
   a.tilesX = (r->W + 7) / 8;
   a.refill = r->p.walk_refill;
   a.walkCtas = r->p.walk_ctas;
@@ -750,13 +795,31 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
   // and is exact for origins within the scene's range
   a.ordered = S.ord && S.traversal == 0 && !a.counting && !r->refWalk && std::fabs(cam->pos[0]) <= S.ordRange &&
               std::fabs(cam->pos[1]) <= S.ordRange && std::fabs(cam->pos[2]) <= S.ordRange;
-  cudaStream_t st = r->st;
+  const bool budgeted = adaptive && r->frame >= r->p.warmup_frames;
+  // an overlapped frame traces beside the one before it and is accumulated
+  // after it; one that starts from the accumulated image waits first
+  if (budgeted) at.slot = 0;
+  const RenderBuffers& rb = at.slot ? r->slot[at.slot - 1] : r->rb;
+  cudaStream_t st = at.slot ? r->stSlot[at.slot - 1] : r->st;
+  const uint32_t prevSlot = r->lastSlot;
+  auto after_previous = [&]() -> cudaError_t {
+    return at.overlap && prevSlot != at.slot ? cudaStreamWaitEvent(st, r->evSlot[prevSlot], 0) : cudaSuccess;
+  };
+  auto finished = [&]() -> gbpt_status {
+    if (at.overlap) CK(cudaEventRecord(r->evSlot[at.slot], st));
+    r->lastSlot = at.slot;
+    return GBPT_OK;
+  };
   // filter-only mode: frames past "Render Iteration" trace nothing and only
   // filter again (src/cudaRTBDPTStreamBilat.cu:1278)
   const uint32_t RI = r->p.render_iterations;
   auto traces = [&](uint32_t f) { return !bilat || RI == 0 || f < RI; };
   r->lastTraced = traces(r->frame);
-  if (!r->lastTraced) return bilat_filter(r, st, timing);
+  if (!r->lastTraced) {
+    CK(after_previous());
+    gbpt_status fs = bilat_filter(r, st, timing);
+    return fs == GBPT_OK ? finished() : fs;
+  }
 
   // plain and PTSC frames can be issued as one CUDA graph (gbpt_renderer_set_graphs)
   const bool useGraph = r->graphs && !a.counting && (r->mode == GBPT_MODE_BDPT_SC || pt);
@@ -792,6 +855,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
   auto launch_ahead = [&]() -> gbpt_status {
     CK(cudaEventRecord(r->evMain, st));
     CK(cudaStreamWaitEvent(r->stLight, r->evMain, 0));
+    if (at.overlap && prevSlot != at.slot) CK(cudaStreamWaitEvent(r->stLight, r->evSlot[prevSlot], 0));
     FrameArgs an = a;
     an.frame = r->frame + k;
     an.cacheSel = nsel;
@@ -805,8 +869,8 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
   // camera rays (or the adaptive budget), the bounce loop, accumulation;
   // tm: phase events between the launches
   auto body = [&](bool tm) -> gbpt_status {
-    const bool budgeted = adaptive && r->frame >= r->p.warmup_frames;
     if (budgeted) {
+      CK(after_previous());
       float delta = r->p.filter_sigma_spatial > 0.f ? r->p.filter_sigma_spatial : r->p.filter_color_eud;
       ensure_gauss(r, delta, r->p.filter_radius);
       CK(launch_bilateral(r->result, r->gpos, r->gnorm, r->p.filter_diffuse ? r->gdiff : nullptr, r->W, r->H,
@@ -852,9 +916,9 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
         CK(launch_walk(S, a, rbx, in, d > 0 ? (int)((d - 1) & 1u) : -1, (int)(d & 1u), d, sx));
         if (aside && d + 1 == K) {
           CK(cudaEventRecord(r->evFork, sx));
-          CK(cudaStreamWaitEvent(r->stBand[0], r->evFork, 0));
-          CK(launch_verify(S, rbx, 0, r->stBand[0]));
-          CK(cudaEventRecord(r->evJoin[0], r->stBand[0]));
+          CK(cudaStreamWaitEvent(r->stBand[at.slot], r->evFork, 0));
+          CK(launch_verify(S, rbx, 0, r->stBand[at.slot]));
+          CK(cudaEventRecord(r->evJoin[at.slot], r->stBand[at.slot]));
         }
         if (mk) mark(r, kPhTrace, tm);
         CK(launch_shade(S, a, rbx, in, d, tailRun && d + 1 == K, sx));
@@ -870,7 +934,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
       }
       if (checks) {
         if (aside)
-          CK(cudaStreamWaitEvent(sx, r->evJoin[0], 0));
+          CK(cudaStreamWaitEvent(sx, r->evJoin[at.slot], 0));
         else if (K > 0)
           CK(launch_verify(S, rbx, 0, sx));
         CK(launch_verify(S, rbx, 1, sx));
@@ -882,10 +946,10 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
     r->lastBands = nb;
     if (budgeted || nb == 1) {
       if (!budgeted) {
-        CK(launch_camera(a, r->rb, st));
+        CK(launch_camera(a, rb, st));
         mark(r, kPhOther, tm);
       }
-      gbpt_status be = bounces(r->rb, st, true);
+      gbpt_status be = bounces(rb, st, true);
       if (be != GBPT_OK) return be;
     } else {
       // one wavefront per band: camera rays and every bounce of the band on its
@@ -904,6 +968,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
       for (uint32_t b = 0; b < nb; b++) CK(cudaStreamWaitEvent(st, r->evJoin[b], 0));
     }
     mark(r, kPhTrace, tm);
+    if (!budgeted) CK(after_previous());
     if (budgeted) {
       if (binary)
         CK(launch_binary_apply(a, r->rb, r->ab, r->result, r->sampleN, r->gpos, r->gnorm, r->gdiff, st));
@@ -911,15 +976,15 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
         CK(launch_adapt_accum(a, r->rb, r->ab, r->result, r->sampleN, r->gpos, r->gnorm, r->gdiff, st));
       mark(r, kPhAdapt, tm);
     } else if (pt) {
-      CK(launch_apply_pt(a, r->rb, r->result, r->sampleN, st));
+      CK(launch_apply_pt(a, rb, r->result, r->sampleN, st));
       mark(r, kPhOther, tm);
     } else if (bilat) {
-      CK(launch_apply_bilat(a, r->rb, r->result, r->sampleN, r->gpos, r->gnorm, r->gdiff, r->gemis, r->direct, r->pot,
+      CK(launch_apply_bilat(a, rb, r->result, r->sampleN, r->gpos, r->gnorm, r->gdiff, r->gemis, r->direct, r->pot,
                             st));
       mark(r, kPhOther, tm);
       return bilat_filter(r, st, tm);
     } else {
-      CK(launch_apply(a, r->rb, r->result, r->sampleN, adaptive ? r->gpos : nullptr, r->gnorm, r->gdiff, st));
+      CK(launch_apply(a, rb, r->result, r->sampleN, adaptive ? r->gpos : nullptr, r->gnorm, r->gdiff, st));
       mark(r, kPhOther, tm);
     }
     return GBPT_OK;
@@ -927,8 +992,12 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
 
   if (!useGraph || !r->graphWarm) {
     if (inlineLight) {
+      CK(after_previous());  // which may still read the cache
       CK(launch_light_pass(S, al, r->rb, st));
+      if (at.overlap) CK(cudaEventRecord(r->evLight[sel], st));
       mark(r, kPhLight, timing);
+    } else if (at.overlap && !pt) {
+      CK(cudaStreamWaitEvent(st, r->evLight[sel], 0));
     }
     if (ahead) {
       gbpt_status e = launch_ahead();
@@ -938,7 +1007,8 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
       prepare_launches();
       r->graphWarm = true;
     }
-    return body(timing);
+    gbpt_status e = body(timing);
+    return e == GBPT_OK ? finished() : e;
   }
   // One graph per frame: captured, then applied to the renderer's executable
   // graph of the same shape (with or without an inline light pass) by
@@ -999,6 +1069,7 @@ gbpt_status read_ctr(gbpt_renderer* r, DevCounters* out) {
     out->nodesS += c[b].nodesS;
     out->trisS += c[b].trisS;
     out->errFlags |= c[b].errFlags;
+    for (int k = 0; k < 2 && b < r->lastSlots; k++) out->checkN[k] = std::max(out->checkN[k], c[b].checkN[k]);
     if (b < r->lastBands) out->paths += c[b].paths;
   }
   return GBPT_OK;
@@ -1028,6 +1099,68 @@ gbpt_status ensure_conn(gbpt_renderer* r) {
   return GBPT_OK;
 }
 
+// Buffers, streams and events of the frames in flight beside the work
+// stream's.  False (the frames then run one after another) when they would
+// take more than 1/32 of the free memory: other renderers keep their room.
+bool ensure_slots(gbpt_renderer* r) {
+  const RenderBuffers& rb = r->rb;
+  if (r->slotMem && r->slotConn != rb.connDepth) {
+    for (cudaStream_t x : r->stSlot) cudaStreamSynchronize(x);
+    dfree(r->slotMem);
+    r->slotMem = nullptr;
+  }
+  const size_t cap = rb.cap;
+  r->slots = frame_slots(cap);
+  for (int pass = r->slotMem ? 1 : 0; pass < 2; pass++) {  // size, then lay out
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+      char* p = r->slotMem + at;
+      at += (bytes + 255) / 256 * 256;
+      return p;
+    };
+    for (uint32_t k = 0; k < r->slots - 1; k++) {
+      RenderBuffers x = rb;
+      for (Wave& w : x.wave) {
+        float4* b = (float4*)take(cap * 64);
+        w = Wave{b, b + cap, b + 2 * cap, b + 3 * cap};
+      }
+      x.hit = (float4*)take((cap + rb.carryCap) * 16);
+      for (float4*& q : x.sh) q = (float4*)take(cap * 48);
+      x.res = (float4*)take(cap * 16);
+      x.gbuf = (float4*)take(cap * 48);
+      x.dsm = (float4*)take(cap * 16);
+      x.slotPix = (uint32_t*)take(cap * 4);
+      x.slotSmp = (uint32_t*)take(cap * 4);
+      for (float4*& q : x.carry) q = (float4*)take((size_t)rb.carryCap * kCarryF4 * 16);
+      x.open = (decltype(x.open))take((size_t)rb.openCap * sizeof(*x.open));
+      x.check = (decltype(x.check))take((size_t)rb.checkCap * 2 * kCheckF4 * sizeof(*x.check));
+      x.fix = (decltype(x.fix))take((size_t)rb.checkCap * 2 * sizeof(*x.fix));
+      x.conn = (decltype(x.conn))take(cap * rb.connDepth * sizeof(*x.conn));
+      x.ctr = rb.ctr + 1 + k;
+      x.lctr = rb.ctr;
+      if (pass) r->slot[k] = x;
+    }
+    if (pass == 0) {
+      size_t freeB = 0, totB = 0;
+      if (cudaMemGetInfo(&freeB, &totB) != cudaSuccess || at > freeB / 32) return false;
+      if (cudaMalloc((void**)&r->slotMem, at) != cudaSuccess) {
+        cudaGetLastError();
+        r->slotMem = nullptr;
+        return false;
+      }
+      r->slotConn = rb.connDepth;
+    }
+  }
+  bool ok = true;
+  if (!r->evCall) ok = cudaEventCreateWithFlags(&r->evCall, cudaEventDisableTiming) == cudaSuccess;
+  for (cudaEvent_t& e : r->evSlot)
+    if (!e) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+  for (cudaStream_t& x : r->stSlot)
+    if (!x) ok = ok && cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
 gbpt_status render_impl(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, uint32_t frames, float* out,
                         int32_t outDev, gbpt_stats* stats) {
   if (!r || !s || !cam) return fail(GBPT_ERR_INVALID_ARG, "NULL renderer, scene or camera");
@@ -1045,12 +1178,31 @@ gbpt_status render_impl(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam,
   }
   const uint64_t launches0 = launch_count();
   r->evs.clear();
+  // frames that do not need each other's image are traced side by side
+  const bool carrying = r->p.carry_steps && !(s->dev.traversal == 1 && s->dev.wide);
+  const bool overlap = frames > 1 && !timing && !r->graphs && !r->counting && !keeps_moments(r) &&
+                       (adaptive_mode(r) || bands_for(r->p.bands, (size_t)r->W * r->H, carrying) == 1) &&
+                       ensure_slots(r);
+  r->lastSlots = overlap ? r->slots : 1;
+  r->lastSlot = 0;
+  if (overlap) {
+    CK(cudaEventRecord(r->evCall, r->st));
+    for (cudaStream_t x : r->stSlot) CK(cudaStreamWaitEvent(x, r->evCall, 0));
+    CK(cudaEventRecord(r->evSlot[0], r->st));
+  }
   for (uint32_t f = 0; f < frames; f++) {
     // NVTX range per frame (free without a profiler attached; ncu --nvtx can filter on it)
     nvtxRangePushA("gbpt frame");
-    stt = frame_once(r, s, cam, timing);
+    FramePlace at;
+    at.overlap = overlap;
+    if (overlap) at.slot = (frames - 1 - f) % r->slots;
+    stt = frame_once(r, s, cam, timing, at);
     nvtxRangePop();
-    if (stt != GBPT_OK) return stt;
+    if (stt != GBPT_OK) {
+      if (overlap)
+        for (cudaStream_t x : r->stSlot) cudaStreamSynchronize(x);
+      return stt;
+    }
   }
   const size_t np = (size_t)r->W * r->H;
   if (out) CK(cudaMemcpyAsync(out, output_view(r), np * 12, outDev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
