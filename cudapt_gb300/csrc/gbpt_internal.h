@@ -29,7 +29,7 @@ std::vector<float> collapse_wide(const HostBVH& bvh);
 // false: the scene keeps the reference's walk (empty children, boxes that are
 // not nested, more than 2^24 nodes, depth, extreme coordinates).  tris: 16
 // words per triangle in BVH order (p0, pad, p1 - p0, pad, p2 - p0, 5 pads).
-bool ordered_tree(const HostBVH& bvh, const float* tris, OrderedTree* out);
+bool ordered_tree(const HostBVH& bvh, OrderedTree* out);
 
 // sqrt(mean((a - b)^2)) over n floats in device memory, summed in double on
 // `stream` (a cudaStream_t); image.cu

@@ -1537,6 +1537,24 @@ __global__ void k_apply_pt(FrameArgs a, RenderBuffers b, float* result, uint32_t
   sampleN[p] = a.frame + 1;  // frames so far (the reference keeps no count in this mode)
 }
 
+// Leaf records of the ordered walk, one thread each: 21 MB that would otherwise
+// be gathered on the host and copied (hall: 332,180 records).
+__global__ void k_ord_leaves(const float4* __restrict__ nodes, const float4* __restrict__ tris,
+                             const uint32_t* __restrict__ bin, uint32_t n, float4* __restrict__ out) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const size_t i = bin[k];
+  const float4 lo = nodes[2 * i], hi = nodes[2 * i + 1];
+  const uint32_t first = __float_as_uint(lo.w), cnt = __float_as_uint(hi.w);
+  const float4 p0 = tris[4 * (size_t)first], e0 = tris[4 * (size_t)first + 1], e1 = tris[4 * (size_t)first + 2];
+  const bool many = cnt != 1u;  // several triangles: the record names them
+  float4* r = out + 4 * (size_t)k;
+  r[0] = make_float4(many ? __uint_as_float(cnt) : p0.x, p0.y, p0.z, e0.x);
+  r[1] = make_float4(e0.y, e0.z, e1.x, e1.y);
+  r[2] = make_float4(e1.z, lo.x, lo.y, lo.z);
+  r[3] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(many ? first | kOrdManyTris : first));
+}
+
 __global__ void k_prob_view(const float* pot, uint32_t np, float minProb, float* out) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= np) return;
@@ -1671,6 +1689,14 @@ cudaError_t launch_light_pass(const DevScene& S, const FrameArgs& a, const Rende
   } else {
     k_light<1, false><<<1, threads, 0, st>>>(S, a, cache, b.cacheCap, b.ctr);
   }
+  note_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_ord_leaves(const float4* nodes, const float4* tris, const uint32_t* bin, uint32_t n, float4* out,
+                              cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  k_ord_leaves<<<(n + kBlock - 1) / kBlock, kBlock, 0, st>>>(nodes, tris, bin, n, out);
   note_launches(1);
   return cudaGetLastError();
 }

@@ -204,6 +204,10 @@ uint32_t tail_from(uint32_t eyeDepth, bool wide, bool ordered, int32_t requested
 // refill threshold of the persistent walks: `requested` when 1..32, else
 // GBPT_WALK_REFILL when set, else 8 (reference order) or 20 (wide order)
 uint32_t walk_refill_for(uint32_t requested, bool wide);
+// The ordered walk's leaf records (ordered.h): record k is binary leaf bin[k]
+// of `nodes` with its first triangle of `tris`.
+cudaError_t launch_ord_leaves(const float4* nodes, const float4* tris, const uint32_t* bin, uint32_t n, float4* out,
+                              cudaStream_t st);
 // Queries (once) the launch shapes of the wavefront kernels, which also loads
 // them: call before the first stream capture.
 void prepare_launches();

@@ -1,7 +1,7 @@
 // Layout of the ordered walk's tree (made by ordered_tree.cpp, walked by ordered.cuh).
 #pragma once
 #include <cstdint>
-#include <vector>
+#include <memory>
 
 namespace gbpt {
 
@@ -16,7 +16,9 @@ constexpr uint32_t kOrdMaxIndex = 1u << 24, kOrdManyTris = 0x80000000u;
 constexpr uint32_t kOrdStack = 20;  // stack entries of a walk: at most one per level below the root
 
 struct OrderedTree {
-  std::vector<float> nodes, leaves;
+  std::unique_ptr<float[]> nodes;      // nodeN x kOrdNodeWords
+  std::unique_ptr<uint32_t[]> leaves;  // binary leaf of each leaf record
+  uint32_t nodeN = 0, leafN = 0;
   float range = 0.f;  // largest |origin coordinate| the walk is exact for
 };
 
