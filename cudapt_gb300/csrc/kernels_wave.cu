@@ -517,7 +517,7 @@ __device__ __forceinline__ void warp_add_u64(unsigned long long* dst, uint32_t v
 // the long ones must start early; then the walks the previous launch carried,
 // then the extension rays (hall 1280x720: 181.4 -> 187.9 Mpaths/s against
 // extension rays first; interior 169.0 -> 168.2).
-// Every ray still visits nodes exactly in TracePrimitive's order, so per-ray
+// Every ray still reaches leaves in TracePrimitive's order, so per-ray
 // results do not depend on this scheduling.  The any-hit walk stops at the
 // first hit closer than maxDist: that is exactly when the reference's
 // closest-hit walk with the same maxDist would report a hit.

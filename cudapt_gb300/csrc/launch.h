@@ -194,9 +194,6 @@ cudaError_t launch_fold(const RenderBuffers& b, cudaStream_t st);
 // starting with the connection attached to each path in queue (t - 1) & 1),
 // then of every walk the bounce launches carried; one lane per path
 cudaError_t launch_tail(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K, cudaStream_t st);
-// first bounce handled by the tail kernel: `requested` when >= 0 (>= D: none),
-// else GBPT_TAIL_FROM when set, else D/2 - 1 (wide order: D/2) for D > 6 and
-// none for D <= 6
 // first bounce the tail kernel carries (requested >= 0, the GBPT_TAIL_FROM
 // override, or the default for the depth cap, the paths of one wavefront and
 // whether the bounce launches carry walks)

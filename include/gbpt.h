@@ -248,7 +248,10 @@ gbpt_status gbpt_get_params(const gbpt_renderer* r, gbpt_params* params);
  * or host destination.  stats may be NULL. */
 gbpt_status gbpt_render(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, float* out_rgb,
                         int32_t out_is_device, gbpt_stats* stats);
-/* Adds `frames` passes without copying (benchmarks / progressive runs). */
+/* Adds `frames` passes without copying (benchmarks / progressive runs).  With
+ * stats NULL, passes that do not start from each other's image are traced side
+ * by side (up to four, in buffers of their own of at most 1/32 of the free
+ * device memory); the image is that of the same passes one call each. */
 gbpt_status gbpt_render_frames(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, uint32_t frames,
                                gbpt_stats* stats);
 /* RTRenderer::GetResult (include/raytracer.h:311): library-owned, page-locked
