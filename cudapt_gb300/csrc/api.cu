@@ -945,7 +945,9 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
     const bool carrying = a.carrySteps && !wideT;
     const size_t np = (size_t)r->W * r->H;
     const uint32_t nb = adaptive ? 1u : bands_for(r->p.bands, np, carrying);
-    const uint32_t K = std::min(tail_from(D, wideT, a.ordered != 0, r->p.tail_from, np / nb, carrying), D);
+    const uint32_t K = std::min(tail_from(D, wideT, a.ordered != 0, r->p.tail_from, np / nb, carrying,
+                                            at.overlap && !pt),
+                                  D);
     const bool tailRun = K < D || carrying || a.tailBelow > 0.f;
     auto bounces = [&](const RenderBuffers& rbx, cudaStream_t sx, bool mk) -> gbpt_status {
       int in = 0;

@@ -1838,7 +1838,8 @@ void prepare_launches() {
   shade_grid();
 }
 
-uint32_t tail_from(uint32_t eyeDepth, bool wide, bool ordered, int32_t requested, size_t paths, bool carrying) {
+uint32_t tail_from(uint32_t eyeDepth, bool wide, bool ordered, int32_t requested, size_t paths, bool carrying,
+                   bool beside) {
   // default for the ordered walk while carrying: a frame with fewer camera paths
   // than 1.5 x the tail grid's lanes (116,736) runs in the tail kernel alone, a
   // larger one hands over at bounce 3D/5 when D > 6, else never.  Measured (ms per
@@ -1847,6 +1848,16 @@ uint32_t tail_from(uint32_t eyeDepth, bool wide, bool ordered, int32_t requested
   // unidirectional 333x217 x 8, D = 10: 0 4.49, 2 5.35, 5 6.19; 500x375 binary, D =
   // 6: 0 10.0, 4 9.40, none 9.64; interior 1024x768, D = 10: 0 4.20, 4 3.06, 5 2.88,
   // 6 2.80, 7 2.80; hall 1280x720, D = 5: 0 4.59, 4 3.06, none 2.94.
+  //
+  // A bidirectional frame traced beside others of its call need not end soon, and
+  // bounce launches use the lanes better: from 3/4 of the tail's lanes (58,368
+  // paths) on, D > 4, the tail starts at (D + 3) / 2.  Measured (ms an image, from 0
+  // / from there): Cornell 256x256 x 16, D = 8 2.49 / 2.12; interior 256x256 x 8, D =
+  // 8 4.74 / 4.10, D = 5 3.94 / 3.57; hall 256x256 x 8, D = 5 4.59 / 3.99; interior
+  // 340x340 x 8, D = 5 5.70 / 4.71.  Below the line from 0 is as good or better
+  // (interior 182x181 x 8, D = 8: 3.48 / 3.57; 256x192, D = 5: 3.37 / 3.35), as it is
+  // for D <= 4 (215x215, D = 4: 2.80 / 3.01) and for unidirectional frames, which
+  // shade little between walks (333x217: 2.89, from 2 3.16, from 6 3.58).
   //
   // default of the node-by-node walk while carrying: a frame with fewer camera paths
   // than the walk grid has lanes hands its paths to the tail kernel from bounce
@@ -1874,7 +1885,9 @@ uint32_t tail_from(uint32_t eyeDepth, bool wide, bool ordered, int32_t requested
   }();
   if (requested >= 0) return (uint32_t)requested;
   if (v == -2 && carrying) {
-    if (ordered && paths < (size_t)tail_grid<false, kWalkOrd>() * kBlock * 3 / 2) return 0u;
+    const size_t lanes = (size_t)tail_grid<false, kWalkOrd>() * kBlock;
+    if (ordered && beside && eyeDepth > 4 && paths >= lanes * 3 / 4 && paths < lanes * 3 / 2) return (eyeDepth + 3) / 2;
+    if (ordered && paths < lanes * 3 / 2) return 0u;
     if (!ordered && paths < walk_lanes()) return std::min(eyeDepth, 2u);
     return eyeDepth > 6 ? (ordered ? eyeDepth * 3 / 5 : eyeDepth / 2) : eyeDepth;
   }

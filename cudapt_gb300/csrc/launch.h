@@ -196,8 +196,10 @@ cudaError_t launch_fold(const RenderBuffers& b, cudaStream_t st);
 cudaError_t launch_tail(const DevScene& S, const FrameArgs& a, const RenderBuffers& b, uint32_t K, cudaStream_t st);
 // first bounce the tail kernel carries (requested >= 0, the GBPT_TAIL_FROM
 // override, or the default for the depth cap, the paths of one wavefront and
-// whether the bounce launches carry walks)
-uint32_t tail_from(uint32_t eyeDepth, bool wide, bool ordered, int32_t requested, size_t paths, bool carrying);
+// whether the bounce launches carry walks; beside: a bidirectional frame that
+// shares the machine with others of its call)
+uint32_t tail_from(uint32_t eyeDepth, bool wide, bool ordered, int32_t requested, size_t paths, bool carrying,
+                   bool beside);
 // refill threshold of the persistent walks: `requested` when 1..32, else
 // GBPT_WALK_REFILL when set, else 8 (reference order) or 20 (wide order)
 uint32_t walk_refill_for(uint32_t requested, bool wide);

@@ -106,7 +106,9 @@ typedef struct gbpt_params {
   int32_t tail_from;        /* first bounce the per-path tail kernel carries (>= the depth cap: none;
                                -1: while carrying, bounce 0 for a frame with fewer camera paths than 1.5 x
                                the tail grid's lanes (2 and the walk grid's where the scene keeps the
-                               reference's walk), else 3/5 of the depth (1/2) when the cap exceeds 6, else none;
+                               reference's walk; (depth + 3) / 2 for a bidirectional frame of at least half as
+                               many, depth > 4, traced beside others of its call), else 3/5 of the depth (1/2)
+                               when the cap exceeds 6, else none;
                                without carrying depth / 2 - 1 (wide order: depth / 2) when the cap
                                exceeds 6, else none) */
   uint32_t bands;           /* wavefronts a frame's camera paths are split into, each on its own stream

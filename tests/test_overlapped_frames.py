@@ -58,3 +58,9 @@ def test_on_the_callers_stream(gbdev):
     st = torch.cuda.Stream()
     _compare(gbdev, "interior", (60, 41), 0, 6, calls=2,
              setup=lambda r: check(load().gbpt_renderer_set_stream(r._h, st.cuda_stream)))
+
+
+@pytest.mark.parametrize("size", [(256, 227), (256, 228), (342, 341), (342, 342)])
+@pytest.mark.parametrize("mode", [0, 3])
+def test_sizes_about_the_tail_start(gbdev, mode, size):
+    _compare(gbdev, "cornell", size, mode, 4)
