@@ -338,13 +338,15 @@ enum Phase { kPhLight = 0, kPhTrace, kPhShade, kPhShadow, kPhFilter, kPhAdapt, k
 // leave half of the machine idle: the mean warp of the tail kernel lives half
 // as long as the longest one (Cornell 256x256 262 of 550 thousand cycles,
 // unidirectional 333x217 image 544 of 1074), and the next frame's paths fill
-// that.  Whole images, 1 / 2 / 3 / 4 frames at once (ms): Cornell 256x256 3.59 /
-// 2.66 / 2.48 / 2.60, unidirectional 333x217 4.15 / 3.04 / 2.91 / 2.89, binary
-// allocator 500x375 9.48 / 8.25 / 7.77 / 7.62, filtered 641x359 6.35 / 5.24 /
-// 5.27 / 4.85, adaptive hall 1280x720 33.4 / 30.7 / 31.1 (its walks fill the
-// machine by themselves): the lines lie between those sizes.
+// that.  Whole images, 1 / 2 / 3 / 4 / 6 frames at once (ms): Cornell 256x256
+// 3.59 / 2.66 / 2.12 / 1.98 / 1.91, unidirectional 333x217 4.15 / 3.04 / 2.90 /
+// 2.86 / 2.85, hall 256x256 x 8 - / 4.65 / 4.11 / 3.85 / 3.87, binary allocator
+// 500x375 9.48 / 8.25 / 7.77 / 7.62 / 7.64, filtered 641x359 6.35 / 5.24 / 5.27 /
+// 4.85 / 4.82: four.  From half a million paths on walks fill the machine by
+// themselves (adaptive hall 1280x720 33.4 / 30.7 / 31.1, filtered hall 900x700 x 6
+// - / 12.4 / 13.0): two.
 constexpr uint32_t kFrameSlots = 4;
-uint32_t frame_slots(size_t paths) { return paths < (1u << 17) ? 3u : paths < (1u << 19) ? kFrameSlots : 2u; }
+uint32_t frame_slots(size_t paths) { return paths < (1u << 19) ? kFrameSlots : 2u; }
 
 struct gbpt_renderer {
   uint32_t W = 0, H = 0;
