@@ -876,7 +876,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
   const uint32_t nsel = sel ^ 1u;
   a.cacheSel = sel;
   r->lastSel = sel;
-  bool inlineLight = false, ahead = false;
+  bool inlineLight = false, ahead = false, lightWait = false;
   // the group's first frame: its light pass (a frame inside a group whose
   // cache is not there -- after a restored checkpoint -- makes it too)
   const uint32_t g0 = r->frame - r->frame % k;
@@ -909,6 +909,21 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
     r->cacheFrame[nsel] = r->frame + k;
     return GBPT_OK;
   };
+  // bounce launch d < K: walk (the walks launch d - 1 carried, the extension
+  // rays of its wave, the shadow rays of launch d - 1), then shade, one launch
+  // each; from K (or the bounce a shading launch switched at): one persistent
+  // kernel per frame carries every remaining path to its end (few paths are
+  // left by then, and per-bounce launches would each wait for their slowest
+  // ray).  Without carrying or a switch on the device and with K = D, the
+  // last launch walks the final connections instead of the tail kernel.
+  const uint32_t D = a.eyeDepth;
+  const bool wideT = S.traversal == 1 && S.wide;
+  const bool carrying = a.carrySteps && !wideT;
+  const size_t np = (size_t)r->W * r->H;
+  const uint32_t nb = adaptive ? 1u : bands_for(r->p.bands, np, carrying);
+  const uint32_t K = std::min(
+      tail_from(D, wideT, a.ordered != 0, r->p.tail_from, np / nb, carrying, at.overlap && !pt), D);
+  const bool tailRun = K < D || carrying || a.tailBelow > 0.f;
   // camera rays (or the adaptive budget), the bounce loop, accumulation;
   // tm: phase events between the launches
   auto body = [&](bool tm) -> gbpt_status {
@@ -935,22 +950,6 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
         CK(launch_adapt_budget(a, r->rb, r->ab, r->result, r->sampleN, r->p.desired_n, st));
       mark(r, kPhAdapt, tm);
     }
-    // bounce launch d < K: walk (the walks launch d - 1 carried, the extension
-    // rays of its wave, the shadow rays of launch d - 1), then shade, one launch
-    // each; from K (or the bounce a shading launch switched at): one persistent
-    // kernel per frame carries every remaining path to its end (few paths are
-    // left by then, and per-bounce launches would each wait for their slowest
-    // ray).  Without carrying or a switch on the device and with K = D, the
-    // last launch walks the final connections instead of the tail kernel.
-    const uint32_t D = a.eyeDepth;
-    const bool wideT = S.traversal == 1 && S.wide;
-    const bool carrying = a.carrySteps && !wideT;
-    const size_t np = (size_t)r->W * r->H;
-    const uint32_t nb = adaptive ? 1u : bands_for(r->p.bands, np, carrying);
-    const uint32_t K = std::min(tail_from(D, wideT, a.ordered != 0, r->p.tail_from, np / nb, carrying,
-                                            at.overlap && !pt),
-                                  D);
-    const bool tailRun = K < D || carrying || a.tailBelow > 0.f;
     auto bounces = [&](const RenderBuffers& rbx, cudaStream_t sx, bool mk) -> gbpt_status {
       int in = 0;
       // walks the frame takes as they ended are checked: the bounce launches'
@@ -966,6 +965,7 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
           CK(cudaEventRecord(r->evJoin[at.slot], r->stBand[at.slot]));
         }
         if (mk) mark(r, kPhTrace, tm);
+        if (lightWait && d == 0) CK(cudaStreamWaitEvent(sx, r->evLight[sel], 0));
         CK(launch_shade(S, a, rbx, in, d, tailRun && d + 1 == K, sx));
         if (mk) mark(r, kPhShade, tm);
         in ^= 1;
@@ -1038,11 +1038,24 @@ gbpt_status frame_once(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam, 
   if (!useGraph || !r->graphWarm) {
     if (inlineLight) {
       CK(after_previous());  // which may still read the cache
-      CK(launch_light_pass(S, al, r->rb, st));
-      if (at.overlap) CK(cudaEventRecord(r->evLight[sel], st));
-      mark(r, kPhLight, timing);
+      if (timing || K == 0) {
+        CK(launch_light_pass(S, al, r->rb, st));
+        if (at.overlap) CK(cudaEventRecord(r->evLight[sel], st));
+        mark(r, kPhLight, timing);
+      } else {
+        // beside the camera rays and the first walks: shading is the first to
+        // read the cache.  Filtered 641x359 image 4.88 -> 4.66 ms, binary 500x375
+        // 7.71 -> 7.61, adaptive hall 30.5 -> 30.1, Cornell 256x256 1.96 -> 1.93
+        // (2.50 -> 2.62 with frames that are one tail kernel: those wait).
+        CK(cudaEventRecord(r->evMain, st));
+        CK(cudaStreamWaitEvent(r->stBand[0], r->evMain, 0));
+        CK(launch_light_pass(S, al, r->rb, r->stBand[0]));
+        CK(cudaEventRecord(r->evLight[sel], r->stBand[0]));
+        lightWait = true;
+      }
     } else if (at.overlap && !pt) {
-      CK(cudaStreamWaitEvent(st, r->evLight[sel], 0));
+      if (K == 0) CK(cudaStreamWaitEvent(st, r->evLight[sel], 0));
+      lightWait = K > 0;
     }
     if (ahead) {
       gbpt_status e = launch_ahead();

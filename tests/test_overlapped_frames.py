@@ -64,3 +64,20 @@ def test_on_the_callers_stream(gbdev):
 @pytest.mark.parametrize("mode", [0, 3])
 def test_sizes_about_the_tail_start(gbdev, mode, size):
     _compare(gbdev, "cornell", size, mode, 4)
+
+
+@pytest.mark.parametrize("params", [dict(), dict(light_every=1), dict(bands=2, carry_steps=0), dict(bands=3)])
+@pytest.mark.parametrize("mode", [0, 1, 3])
+def test_light_pass_beside_the_first_walks(gbdev, mode, params):
+    """Calls of one frame without statistics start their bounce launches while the light pass runs."""
+    (v, t, m), cam = scene_arrays("interior")
+    p = gbdev.default_params(eye_depth_max=5, light_depth_max=4, warmup_frames=3, filter_radius=2, bilat_radius=2,
+                             tail_from=5, **params)
+    s = gbdev.RTScene(v, t, m).build_bvh()
+    a, b = (gbdev.RTRenderer(70, 51, mode, p) for _ in range(2))
+    for k in range(8):
+        moved = dict(cam, fov=cam["fov"] * (1.0 + 0.01 * (k // 4)))
+        a.render_frames(s, moved, 1, stats=True)
+        b.render_frames(s, moved, 1, stats=False)
+        for what in (0, 6):
+            assert_bits_equal(b.read_buffer(what), a.read_buffer(what), f"buffer {what} after frame {k}")
