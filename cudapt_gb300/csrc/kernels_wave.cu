@@ -1375,7 +1375,7 @@ __global__ void __launch_bounds__(kCapThreads) k_again(DevScene S, FrameArgs a, 
   }
 }
 
-// ... and of caller-supplied rays (k_trace_rays marks them with triangle -2):
+// ... and of caller-supplied rays (marked with triangle -2 by their kernel):
 // a block looks through 256 rays and answers the marked ones.
 __global__ void __launch_bounds__(kCapThreads) k_resolve_rays(DevScene S, const float* rays, uint32_t n, float maxDist,
                                                               float eps, float* t, int32_t* tri, float* w, float* u,
@@ -1565,6 +1565,72 @@ __global__ void k_prob_view(const float* pot, uint32_t np, float minProb, float*
 }
 
 // ---------------------------------------------------------------------------
+// Caller-supplied rays by the ordered walk: a warp owns `chunk` of them (a
+// multiple of 32), a lane takes the warp's next ray as its walk ends, and the
+// warp's walks step together.  Bound like the bounce launches' walks, by issue;
+// with a thread a ray (k_trace_rays) a warp waits for the longest of its 32
+// walks.  A fixed share needs no counter in memory, and some 200 rays a warp even
+// out.  A million rays in the hall 1.06 -> 0.85 ms.
+__global__ void __launch_bounds__(kBlock, 4) k_trace_ord(DevScene S, const float* rays, uint32_t n, uint32_t chunk,
+                                                         float maxDist, float eps, float* t, int32_t* tri, float* w,
+                                                         float* u, float* v) {
+  __shared__ uint32_t openN;
+  if (threadIdx.x == 0) openN = 0;
+  __syncthreads();
+  const uint64_t first = (uint64_t)(blockIdx.x * (kBlock / 32) + threadIdx.x / 32) * chunk;
+  if (first >= n) return;
+  uint32_t next = (uint32_t)first;
+  const uint32_t end = (uint32_t)min(first + chunk, (uint64_t)n);
+  OrdWalk wk;
+  uint2 stack[kOrdStack];
+  wk.any = false;
+  wk.eps = eps;
+  bool has = false;
+  uint32_t item = 0;
+  for (;;) {
+    wk.stop_long();
+    const uint32_t idle = __ballot_sync(0xffffffffu, !has);
+    if (next < end) {
+      const uint32_t off = __popc(idle & lanemask_lt()), left = end - next;
+      if (!has && off < left) {
+        item = next + off;
+        has = true;
+        const float* r = rays + 6 * (size_t)item;
+        wk.init(S, mk(r[0], r[1], r[2]), mk(r[3], r[4], r[5]), maxDist);
+      }
+      next += min((uint32_t)__popc(idle), left);
+    } else if (idle == 0xffffffffu) {
+      break;
+    }
+#pragma unroll 1
+    for (int k = 0; k < walk_steps<kWalkOrd>(); k++) {
+      if (!wk.step_warp(S, stack, has)) continue;
+      has = false;
+      bool hit = wk.hit();
+      TraceHit h;
+      h.t = wk.minT;
+      h.tri = wk.best;
+      h.w = 1.f - wk.bu - wk.bv;
+      h.u = wk.bu;
+      h.v = wk.bv;
+      if (wk.capped()) {
+        // one in 64 of a block's rays waits for k_resolve_rays, more take the reference's walk
+        if (atomicAdd(&openN, 1u) < chunk / 8u) {
+          tri[item] = -2;
+          continue;
+        }
+        uint32_t nn = 0, nt = 0;
+        hit = trace_ref<false, false>(S, wk.o, wk.d, maxDist, eps, false, h, nn, nt);
+      }
+      t[item] = hit ? h.t : -1.f;
+      tri[item] = hit ? (int32_t)h.tri : -1;
+      w[item] = hit ? h.w : 0.f;
+      u[item] = hit ? h.u : 0.f;
+      v[item] = hit ? h.v : 0.f;
+    }
+  }
+}
+
 // Stand-alone TracePrimitive for caller-supplied rays.
 template <bool kCount>
 __global__ void k_trace_rays(DevScene S, const float* rays, uint32_t n, float maxDist, float eps, int cullback,
@@ -1953,21 +2019,35 @@ cudaError_t launch_trace_rays(const DevScene& S, const float* rays, uint32_t n, 
                               float* t, int32_t* tri, float* w, float* u, float* v, uint32_t* nodes,
                               uint32_t* trisTested, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  uint32_t grid = (n + kBlock - 1) / kBlock;
-  if (nodes && trisTested)
-    k_trace_rays<true><<<grid, kBlock, 0, st>>>(S, rays, n, maxDist, eps, cullback, t, tri, w, u, v, nodes,
-                                                  trisTested);
-  else
-    k_trace_rays<false><<<grid, kBlock, 0, st>>>(S, rays, n, maxDist, eps, cullback, t, tri, w, u, v, nodes,
-                                                   trisTested);
-  note_launches(1);
-  if (!(nodes && trisTested) && S.ord && S.traversal == 0 && !cullback) {
+  const uint32_t grid = n / kBlock + (n % kBlock != 0u);
+  const bool ordered = !(nodes && trisTested) && S.ord && S.traversal == 0 && !cullback;
+  if (ordered) {
+    // Shares from two rays a lane of the grid on (311,296): at 400,000 rays hall
+    // 0.56 -> 0.50 ms, interior 0.42 -> 0.37, at 1,500,000 1.43 -> 0.98 and 1.17 ->
+    // 0.69; at 160,000, where no lane gets a second ray, a thread a ray takes 0.35
+    // against 0.38.  Walks of trees of up to 2048 nodes are short and alike: Cornell
+    // at 400,000 0.068 against 0.076 ms, at 1,500,000 even.
+    static const uint32_t full = grid_for((const void*)k_trace_ord);
+    if (n >= 2u * full * kBlock && S.nodeN > kPopCap) {
+      const uint32_t warps = full * (kBlock / 32), chunk = ((n - 1) / warps / 32 + 1) * 32;
+      k_trace_ord<<<full, kBlock, 0, st>>>(S, rays, n, chunk, maxDist, eps, t, tri, w, u, v);
+    } else {
+      k_trace_rays<false><<<grid, kBlock, 0, st>>>(S, rays, n, maxDist, eps, cullback, t, tri, w, u, v, nodes,
+                                                     trisTested);
+    }
+    note_launches(1);
     const cudaError_t e = cap_launchable(k_resolve_rays);
     if (e != cudaSuccess) return e;
     k_resolve_rays<<<std::min<uint32_t>(grid, cap_grid()), kCapThreads, sizeof(CapShared), st>>>(
         S, rays, n, maxDist, eps, t, tri, w, u, v);
-    note_launches(1);
+  } else if (nodes && trisTested) {
+    k_trace_rays<true><<<grid, kBlock, 0, st>>>(S, rays, n, maxDist, eps, cullback, t, tri, w, u, v, nodes,
+                                                  trisTested);
+  } else {
+    k_trace_rays<false><<<grid, kBlock, 0, st>>>(S, rays, n, maxDist, eps, cullback, t, tri, w, u, v, nodes,
+                                                   trisTested);
   }
+  note_launches(1);
   return cudaGetLastError();
 }
 
