@@ -297,7 +297,12 @@ __global__ void __launch_bounds__(1024) k_light(DevScene S, FrameArgs a, float4*
     if (first) store_lv(cache + 6 * (size_t)x, v);
   }
   uint32_t size = (S.lightN > 0) ? NL : 0;
-  __syncthreads();
+  // the cluster's blocks must all have started before one of them stores to
+  // another's shared memory: co-scheduling alone does not promise it
+  if constexpr (kLanes > 1)
+    cooperative_groups::this_cluster().sync();
+  else
+    __syncthreads();
   for (uint32_t round = 0;; round++) {
     uint32_t bal = __ballot_sync(0xffffffffu, alive && first);
     if (lane == 0) warpCnt[warp] = __popc(bal);
