@@ -61,6 +61,12 @@ __device__ __forceinline__ float byte_float(uint32_t w) {
 
 constexpr uint32_t kPopCap = 2048;          // BVH_TRACE_MAX (include/cudaRTCommon.h:14)
 constexpr uint32_t kPopStop = 4 * kPopCap;  // a bound this large ends a walk early, unresolved
+// Longest direction component the node test takes.  A plane step is cell /
+// (|d| * limit), with cells of at least 2^-24 of the largest coordinate (itself
+// at least 2^-10) and limits of at most 2^67: 2^-141 at this length.  The test's
+// three roundings to subnormal numbers, 2^-150 each, stay below the 2^-7.4
+// cells the planes' margin has left; from 2^92 on the products are zero.
+constexpr float kOrdMaxDir = 0x1p40f;
 
 // Walk state: the current group (child base and inner mask, leaf base and the
 // mask of children still to visit, lowest bit first) in registers, groups with
@@ -93,8 +99,10 @@ struct OrdWalk {
     // no finite direction at all: every slab distance is NaN and the reference's
     // root test fails
     if (isnan(inv.x) && isnan(inv.y) && isnan(inv.z)) gB = 0u;
-    // an origin outside the range the planes' margin covers, or a NaN: unresolved
-    else if (!(fabsf(o.x) <= r && fabsf(o.y) <= r && fabsf(o.z) <= r) || isnan(inv.x + inv.y + inv.z))
+    // an origin outside the range the planes' margin covers, a direction longer
+    // than the node test's products carry, or a NaN: unresolved
+    else if (!(fabsf(o.x) <= r && fabsf(o.y) <= r && fabsf(o.z) <= r) || isnan(inv.x + inv.y + inv.z) ||
+             fmax3_(fabsf(d.x), fabsf(d.y), fabsf(d.z)) > kOrdMaxDir)
       gB = 0u, bound = kPopStop;
   }
 
