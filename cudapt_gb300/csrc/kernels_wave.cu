@@ -1388,13 +1388,14 @@ __global__ void __launch_bounds__(kCapThreads) k_resolve_rays(DevScene S, const 
   extern __shared__ float4 capMem[];
   CapShared& c = *reinterpret_cast<CapShared*>(capMem);
   __shared__ uint32_t list[kCapThreads], count;
-  for (uint32_t base = blockIdx.x * kCapThreads; base < n; base += gridDim.x * kCapThreads) {
-    const uint32_t i = base + threadIdx.x;
+  // 64 bits: the step past the last ray can leave 32
+  for (uint64_t base = (uint64_t)blockIdx.x * kCapThreads; base < n; base += (uint64_t)gridDim.x * kCapThreads) {
+    const uint64_t i = base + threadIdx.x;
     const bool open = i < n && tri[i] == -2;
     if (!__syncthreads_or(open)) continue;
     if (threadIdx.x == 0) count = 0;
     __syncthreads();
-    if (open) list[atomicAdd(&count, 1u)] = i;
+    if (open) list[atomicAdd(&count, 1u)] = (uint32_t)i;
     __syncthreads();
     const uint32_t m = count;
     for (uint32_t k = 0; k < m; k++) {
