@@ -953,6 +953,10 @@ static int bilateral_quo(float c2) {
   if (!(c2 >= 0x1p-40f && c2 <= 0x1p40f)) return kQuoDiv;
   return std::fabs((double)(1.f / c2) * (double)c2 - 1.0) <= 0x1p-25 ? kQuoOnce : kQuoTwice;  // exact in double
 }
+// a product whose divisor is outside the quotient's range: it cannot be taken as a
+// quotient where the other planes are (from 2^121 on 128 * c2 is infinite and an
+// infinite distance gave NaN in place of weight 0)
+static bool product_only(float c2) { return c2 < 0.f && !(c2 <= -0x1p-40f && c2 >= -0x1p40f); }
 
 cudaError_t launch_bilateral(const float* color, const float* pos, const float* norm, const float* emit, uint32_t W,
                              uint32_t H, float ceud, float peud, float neud, float eeud, uint32_t radius,
@@ -967,10 +971,13 @@ cudaError_t launch_bilateral(const float* color, const float* pos, const float* 
   if (smem <= 200 * 1024) {
     // the cases worth a kernel of their own: products throughout, products but for
     // the colour plane (the adaptive modes' defaults), quotients throughout (a
-    // product is the quotient by the same c2 as well); else the division
+    // product is the quotient by the same c2 as well, within the quotient's range);
+    // else the division
     const int qc = bilateral_quo(cc2);
     int qo = std::max(bilateral_quo(pc2), bilateral_quo(nc2));
     if (emit) qo = std::max(qo, bilateral_quo(ec2));
+    const bool divide = qo == kQuoDiv || qc == kQuoDiv || product_only(cc2) || product_only(pc2) ||
+                        product_only(nc2) || (emit && product_only(ec2));
     auto tile = [&](auto kern, auto div) {
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       kern<<<grid, block, smem, st>>>(color, pos, norm, emit, W, H, div(cc2), div(pc2), div(nc2), div(ec2), r, g, out);
@@ -981,7 +988,7 @@ cudaError_t launch_bilateral(const float* color, const float* pos, const float* 
       const auto quo = [](float c2) { return bilateral_div(c2 < 0.f ? -1.f / c2 : c2); };
       if (qo == kQuoMul && qc == kQuoMul) tile(k_bilateral_tile<kE, kRr, kQuoMul, kQuoMul>, bilateral_div);
       else if (qo == kQuoMul && qc == kQuoOnce) tile(k_bilateral_tile<kE, kRr, kQuoOnce, kQuoMul>, bilateral_div);
-      else if (qo == kQuoDiv || qc == kQuoDiv) tile(k_bilateral_tile<kE, kRr, kQuoDiv, kQuoDiv>, bilateral_div);
+      else if (divide) tile(k_bilateral_tile<kE, kRr, kQuoDiv, kQuoDiv>, bilateral_div);
       else tile(k_bilateral_tile<kE, kRr, kQuoTwice, kQuoTwice>, quo);
     };
     using std::integral_constant;
