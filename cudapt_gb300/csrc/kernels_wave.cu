@@ -911,7 +911,7 @@ __device__ __forceinline__ void shade_path(const DevScene& S, const FrameArgs& a
     return;
   }
   io.cont = true;
-  b.conn[(size_t)depth * b.cap + slot] = make_float4(0.f, 0.f, 0.f, 0.f);  // none, until a connection walk says
+  b.conn[(size_t)depth * b.cap + slot] = make_float4(0.f, 0.f, 0.f, 0.f);  // no connection made
   outMul = vmul(outMul, B.lmt);
   io.o = st4u(B.nOrig, slot);
   io.d = st4u(B.nDir, pix);
@@ -938,6 +938,7 @@ __device__ __forceinline__ void shade_path(const DevScene& S, const FrameArgs& a
   f3 c = vmax0(shading(-1.f * dir, irradDir, irrad, B.nl, m.diff, m.metal, m.rough, m.spec, 1.f - m.trans, 1.f));
   if (length(c) > 0.f) {
     io.conn = true;
+    reinterpret_cast<float*>(b.conn + (size_t)depth * b.cap + slot)[3] = -1.f;  // occluded, until its walk says
     io.shA = st4u(pos, slot);
     io.shB = st4(toDir, toDist - kBias);
     const f3 cw = vmul(c, inMul);
@@ -1295,7 +1296,7 @@ __global__ void __launch_bounds__(kCapThreads) k_verify(DevScene S, RenderBuffer
     if (any) {
       if (hit != was) {
         const float4 C = r[2];
-        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 none = make_float4(0.f, 0.f, 0.f, -1.f);
         b.conn[(size_t)__float_as_uint(C.w) * b.cap + __float_as_uint(A.w)] = hit ? none : make_float4(C.x, C.y, C.z, 1.f);
       }
     } else if (got.x == -2.f || hit != was || (hit && (c.answer.x != got.x || __float_as_uint(c.answer.y) != __float_as_uint(got.y)))) {
@@ -1317,7 +1318,7 @@ __global__ void __launch_bounds__(kCapThreads) k_again(DevScene S, FrameArgs a, 
   const uint32_t n = b.ctr->fixN;
   const uint32_t cacheSize = b.lctr->cacheSize[a.cacheSel];
   const float4* __restrict__ cache = b.cache[a.cacheSel];
-  uint32_t extRays = 0, shRays = 0;
+  int32_t extRays = 0, shRays = 0;
   // the answer of one ray, for every thread; (-1, ...) on a miss
   auto walk = [&](float4 o, float4 d, float far, bool any) {
     OrdWalk w;
@@ -1348,6 +1349,14 @@ __global__ void __launch_bounds__(kCapThreads) k_again(DevScene S, FrameArgs a, 
       skip |= __float_as_uint(q[0].w) == __float_as_uint(io.o.w) && __float_as_uint(q[3].w) < __float_as_uint(io.s.w);
     }
     if (skip) continue;  // block-uniform
+    // the rays of the continuation that was wrong come off the counters: one per
+    // bounce up to its end, one per connection it made.  (Paths that waited for
+    // this answer have none.)
+    if (!(a.bilat || a.moments)) {
+      const uint32_t slot = __float_as_uint(io.o.w), from = __float_as_uint(io.s.w), end = __float_as_uint(b.res[slot].w);
+      extRays -= (int32_t)(end - from);
+      for (uint32_t d = from; d < end; d++) shRays -= b.conn[(size_t)d * b.cap + slot].w != 0.f ? 1 : 0;
+    }
     if (a.gbuffer && threadIdx.x == 0 && __float_as_uint(io.s.w) == 0u) {  // as k_camera leaves them
       float4* g = b.gbuf + 3 * (size_t)__float_as_uint(io.o.w);
       g[0] = g[1] = g[2] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1374,9 +1383,9 @@ __global__ void __launch_bounds__(kCapThreads) k_again(DevScene S, FrameArgs a, 
       extRays++;
     }
   }
-  if (threadIdx.x == 0 && extRays) {
-    atomicAdd(&b.ctr->rays, (unsigned long long)(extRays + shRays));
-    atomicAdd(&b.ctr->shadowRays, (unsigned long long)shRays);
+  if (threadIdx.x == 0 && (extRays || shRays)) {  // (negative: the sums wrap to the right value)
+    atomicAdd(&b.ctr->rays, (unsigned long long)(long long)(extRays + shRays));
+    atomicAdd(&b.ctr->shadowRays, (unsigned long long)(long long)shRays);
   }
 }
 
@@ -1432,7 +1441,7 @@ __global__ void k_fold(RenderBuffers b) {
   uint32_t n = 0;
   for (uint32_t d = 0; d < k; d++) {
     const float4 c = b.conn[(size_t)d * b.cap + s];
-    if (c.w != 0.f) {
+    if (c.w > 0.f) {
       x = x + c.x;
       y = y + c.y;
       z = z + c.z;

@@ -154,7 +154,7 @@ struct RenderBuffers {
   uint32_t checkCap;
   // per bounce d < connDepth and slot (index d * cap + slot): the connection
   // the path made at bounce d, contribution.xyz and .w = 1 when its walk found
-  // it unoccluded, 0 when occluded or none was made; k_fold sums them into the
+  // it unoccluded, -1 when occluded, 0 when none was made; k_fold sums them into the
   // slot's result in bounce order once the frame's walks are done.  Until
   // then a slot's res word holds the path's emission at its end and, in .w,
   // the bounce it ended at.
