@@ -1611,7 +1611,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_ord(DevScene S, const float
         item = next + off;
         has = true;
         const float* r = rays + 6 * (size_t)item;
-        wk.init(S, mk(r[0], r[1], r[2]), mk(r[3], r[4], r[5]), maxDist);
+        wk.init_caller(S, mk(r[0], r[1], r[2]), mk(r[3], r[4], r[5]), maxDist);
       }
       next += min((uint32_t)__popc(idle), left);
     } else if (idle == 0xffffffffu) {

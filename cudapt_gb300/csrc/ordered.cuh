@@ -61,7 +61,7 @@ __device__ __forceinline__ float byte_float(uint32_t w) {
 
 constexpr uint32_t kPopCap = 2048;          // BVH_TRACE_MAX (include/cudaRTCommon.h:14)
 constexpr uint32_t kPopStop = 4 * kPopCap;  // a bound this large ends a walk early, unresolved
-// Longest direction component the node test takes.  A plane step is cell /
+// Longest direction component the node test takes (init_caller).  A plane step is cell /
 // (|d| * limit), with cells of at least 2^-24 of the largest coordinate (itself
 // at least 2^-10) and limits of at most 2^67: 2^-141 at this length.  The test's
 // three roundings to subnormal numbers, 2^-150 each, stay below the 2^-7.4
@@ -99,11 +99,16 @@ struct OrdWalk {
     // no finite direction at all: every slab distance is NaN and the reference's
     // root test fails
     if (isnan(inv.x) && isnan(inv.y) && isnan(inv.z)) gB = 0u;
-    // an origin outside the range the planes' margin covers, a direction longer
-    // than the node test's products carry, or a NaN: unresolved
-    else if (!(fabsf(o.x) <= r && fabsf(o.y) <= r && fabsf(o.z) <= r) || isnan(inv.x + inv.y + inv.z) ||
-             fmax3_(fabsf(d.x), fabsf(d.y), fabsf(d.z)) > kOrdMaxDir)
+    // an origin outside the range the planes' margin covers, or a NaN: unresolved
+    else if (!(fabsf(o.x) <= r && fabsf(o.y) <= r && fabsf(o.z) <= r) || isnan(inv.x + inv.y + inv.z))
       gB = 0u, bound = kPopStop;
+  }
+  // A caller's ray: its direction may also be longer than the node test's products
+  // carry.  The renderer's directions are quotients by their own length (or not
+  // finite) and skip the test: 1 % of a hall pass.
+  __device__ __forceinline__ void init_caller(const DevScene& S, gb::f3 o_, gb::f3 d_, float maxDist) {
+    init(S, o_, d_, maxDist);
+    if (fmax3_(fabsf(d.x), fabsf(d.y), fabsf(d.z)) > kOrdMaxDir) gB = 0u, bound = kPopStop;
   }
 
   // a limit above 1e20 lies beyond every plane (coordinates up to 1e9, slopes
@@ -691,7 +696,7 @@ __device__ __forceinline__ bool trace_ord(const DevScene& S, gb::f3 o, gb::f3 d,
   uint2 stack[kOrdStack];
   w.any = false;
   w.eps = eps;
-  w.init(S, o, d, maxDist);
+  w.init_caller(S, o, d, maxDist);
   while (!w.step(S, stack)) {
   }
   if (w.capped()) {
