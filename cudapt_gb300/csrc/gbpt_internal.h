@@ -27,8 +27,9 @@ bool build_bvh(const gbpt_vertex* verts, const gbpt_triangle* tris, uint32_t nt,
 std::vector<float> collapse_wide(const HostBVH& bvh);
 
 // false: the scene keeps the reference's walk (empty children, boxes that are
-// not nested, more than 2^24 nodes, depth, extreme coordinates).  tris: 16
-// words per triangle in BVH order (p0, pad, p1 - p0, pad, p2 - p0, 5 pads).
+// not nested, more than 2^24 nodes, depth, extreme coordinates, leaves small
+// against the scene's distance from the origin).  The leaf records are filled in
+// on the device (launch_ord_leaves).
 bool ordered_tree(const HostBVH& bvh, OrderedTree* out);
 
 // sqrt(mean((a - b)^2)) over n floats in device memory, summed in double on
