@@ -253,11 +253,19 @@ gbpt_status upload_ordered(gbpt_scene* s, OrderedJob& job) {
   cudaError_t e = cudaMemcpy(bin, t.leaves.get(), (size_t)t.leafN * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = launch_ord_leaves(s->dNodes, s->dTris, bin, t.leafN, s->dOrdLeaf, nullptr);
   if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  DevScene dev = s->dev;
+  dev.ord = s->dOrd;
+  dev.ordLeaf = s->dOrdLeaf;
+  dev.ordRange = t.range;
+  const bool keep = e == cudaSuccess && !walks_pass_bound(dev, bin, nullptr, &e);
   dfree(bin);
   CK(e);
-  s->dev.ord = s->dOrd;
-  s->dev.ordLeaf = s->dOrdLeaf;
-  s->dev.ordRange = t.range;
+  if (keep) {
+    s->dev = dev;
+  } else {
+    dfree(s->dOrd);
+    dfree(s->dOrdLeaf);
+  }
   return GBPT_OK;
 }
 

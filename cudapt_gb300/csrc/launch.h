@@ -207,6 +207,9 @@ uint32_t walk_refill_for(uint32_t requested, bool wide);
 // of `nodes` with its first triangle of `tris`.
 cudaError_t launch_ord_leaves(const float4* nodes, const float4* tris, const uint32_t* bin, uint32_t n, float4* out,
                               cudaStream_t st);
+// Whether too many walks of a scene with an ordered tree pass the reference's pop
+// bound for the ordered walk to pay (waits for the stream; word: scratch).
+bool walks_pass_bound(const DevScene& S, uint32_t* word, cudaStream_t st, cudaError_t* err);
 // Queries (once) the launch shapes of the wavefront kernels, which also loads
 // them: call before the first stream capture.
 void prepare_launches();

@@ -4,6 +4,7 @@ tail kernel from the first bounce to none, without carrying, and with the
 learned allocator's statistics kept.  The oracle's image, word for word."""
 import functools
 
+import numpy as np
 import pytest
 
 from helpers import assert_bits_equal, camera_rays
@@ -16,10 +17,25 @@ SIZES = [(61, 37), (16, 9)]  # more such walks than the lists hold, and fewer
 
 @functools.lru_cache(maxsize=None)
 def _scene():
+    """The sticks in a space so large that few of its rays meet them: it gets the ordered walk's tree."""
     import cudapt_gb300 as gb
     (v, t, m), cam = _sticks(6000)
+    far = np.zeros(6, v.dtype)
+    far["pos"] = np.repeat(np.float32([[-150.0], [160.0]]), 3, 0) + np.tile(np.eye(3, dtype=np.float32), (2, 1))
+    far["norm"] = (0.0, 1.0, 0.0)
+    ft = np.zeros(2, t.dtype)
+    for k, name in enumerate(("v0", "v1", "v2")):
+        ft[name] = len(v) + np.array([k, 3 + k])
+    v, t = np.concatenate([v, far]), np.concatenate([t, ft])
     s = gb.RTScene(v, t, m).build_bvh()
     assert (s.trace_rays(camera_rays(cam, *SIZES[0], 1), counts=True, eps=1e-4)["nodes"] == 2048).sum() > 100
+    launches = []
+    for counting in (True, False):  # the ordered walk adds three launches that check its answers
+        r = gb.RTRenderer(8, 8, 0, _params(tail_from=2))
+        r.set_counting(counting)
+        r.render(s, cam)
+        launches.append(r.last_stats["launches"])
+    assert launches[1] == launches[0] + 3
     return s, (v, t, m), cam
 
 
@@ -71,3 +87,14 @@ def test_statistics_of_the_learned_allocator(gbdev, size, mode, tail_from):
         got.append([r.read_buffer(k) for k in (0, 6, 11, 12)])
     for a, b, what in zip(*got, ("image", "sampleN", "second moments", "path lengths")):
         assert_bits_equal(b, a, what)
+
+
+@pytest.mark.parametrize("size", [(64, 47), (672, 464)], ids=str)  # a thread a ray, and shared out over warps
+def test_rays_past_the_bound(gbdev, size):
+    s, _, cam = _scene()
+    rays = camera_rays(cam, *size, 3)
+    for kw in (dict(eps=1e-4), dict(), dict(max_dist=40.0, eps=1e-4)):
+        want, got = s.trace_rays(rays, counts=True, **kw), s.trace_rays(rays, **kw)
+        assert (want["nodes"] == 2048).mean() > 0.01
+        for k in ("tri", "t", "w", "u", "v"):
+            assert_bits_equal(got[k], want[k], f"{size} {kw} {k}")
