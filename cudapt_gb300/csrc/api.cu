@@ -1135,7 +1135,10 @@ gbpt_status read_ctr(gbpt_renderer* r, DevCounters* out) {
     out->nodesS += c[b].nodesS;
     out->trisS += c[b].trisS;
     out->errFlags |= c[b].errFlags;
-    for (int k = 0; k < 2 && b < r->lastSlots; k++) out->checkN[k] = std::max(out->checkN[k], c[b].checkN[k]);
+    if (b < std::max(r->lastSlots, r->lastBands)) {
+      for (int k = 0; k < 2; k++) out->checkN[k] = std::max(out->checkN[k], c[b].checkN[k]);
+      out->openOver |= c[b].openOver;
+    }
     if (b < r->lastBands) out->paths += c[b].paths;
   }
   return GBPT_OK;
@@ -1249,7 +1252,7 @@ gbpt_status render_impl(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam,
   const bool overlap = frames > 1 && !timing && !r->graphs && !r->counting && !keeps_moments(r) &&
                        (adaptive_mode(r) || bands_for(r->p.bands, (size_t)r->W * r->H, carrying) == 1) &&
                        ensure_slots(r);
-  r->lastSlots = overlap ? r->slots : 1;
+  r->lastSlots = overlap ? std::min(r->slots, frames) : 1;
   r->lastSlot = 0;
   if (overlap) {
     CK(cudaEventRecord(r->evCall, r->st));
@@ -1282,7 +1285,8 @@ gbpt_status render_impl(gbpt_renderer* r, gbpt_scene* s, const gbpt_camera* cam,
     if (stt != GBPT_OK) return stt;
     flags = c.errFlags;
     // most walks of this view run out of pops: the node-by-node walk is the faster one
-    if (c.checkN[0] > r->rb.checkCap || c.checkN[1] > r->rb.checkCap) r->refWalk = true;
+    const uint32_t listed = r->rb.checkCap / r->lastBands;  // a band has its part of the lists
+    if (c.checkN[0] > listed || c.checkN[1] > listed || c.openOver) r->refWalk = true;
     if (flags) {
       for (uint32_t b = 0; b < kMaxBands; b++) CK(cudaMemsetAsync(&r->rb.ctr[b].errFlags, 0, 4, r->st));
       CK(cudaStreamSynchronize(r->st));

@@ -333,7 +333,7 @@ __global__ void k_scan_blocks(uint32_t* blockSum, uint32_t nb, uint32_t gen, Dev
     ctr->fetchT = 0;
     ctr->carryN[0] = ctr->carryN[1] = ctr->carryN[2] = 0;
     ctr->fetchTail = 0;
-    ctr->openN = ctr->checkN[0] = ctr->checkN[1] = ctr->fixN = 0;
+    ctr->openN = ctr->openOver = ctr->checkN[0] = ctr->checkN[1] = ctr->fixN = 0;
     ctr->tailAt = 0xFFFFFFFFu;
   }
 }
@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_bin_search(FrameArgs a, Render
     b.ctr->fetchT = 0;
     b.ctr->carryN[0] = b.ctr->carryN[1] = b.ctr->carryN[2] = 0;
     b.ctr->fetchTail = 0;
-    b.ctr->openN = b.ctr->checkN[0] = b.ctr->checkN[1] = b.ctr->fixN = 0;
+    b.ctr->openN = b.ctr->openOver = b.ctr->checkN[0] = b.ctr->checkN[1] = b.ctr->fixN = 0;
     b.ctr->tailAt = 0xFFFFFFFFu;
   }
 }

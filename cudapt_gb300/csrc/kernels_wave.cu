@@ -457,7 +457,7 @@ __global__ void k_camera(FrameArgs a, RenderBuffers b) {
     b.ctr->fetchT = 0;
     b.ctr->carryN[0] = b.ctr->carryN[1] = b.ctr->carryN[2] = 0;
     b.ctr->fetchTail = 0;
-    b.ctr->openN = b.ctr->checkN[0] = b.ctr->checkN[1] = b.ctr->fixN = 0;
+    b.ctr->openN = b.ctr->openOver = b.ctr->checkN[0] = b.ctr->checkN[1] = b.ctr->fixN = 0;
     b.ctr->tailAt = 0xFFFFFFFFu;
   }
   if (i >= b.count) return;
@@ -799,6 +799,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(DevScene S, RenderBuffers b,
               open = k < b.openCap;
               now = !open;
               if (open) b.open[k] = item | (res ? kOpenCarried : any ? kOpenShadow : 0u);
+              else b.ctr->openOver = 1u;
             } else if (later == kOpenCheck) {
               now = w.bound >= kPopStop;  // an unfinished walk has no answer to take
             }

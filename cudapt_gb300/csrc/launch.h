@@ -64,6 +64,7 @@ struct DevCounters {
   uint32_t carryN[3];     // extension walks carried out of bounce launch L, in counter L % 3
   uint32_t fetchTail;     // next item handed to a lane by the tail kernel
   uint32_t openN;         // walks of this launch listed for k_resolve
+  uint32_t openOver;      // a launch of the frame found that list full
   uint32_t checkN[2];     // walks of the bounce launches / the tail kernel recorded for k_verify
   uint32_t fixN;          // of those, paths to run again
   uint32_t tailAt;        // bounce from which the tail kernel carries the frame's paths, when a shading
