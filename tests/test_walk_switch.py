@@ -54,3 +54,24 @@ def test_full_lists_of_walks_that_wait(gbdev, collect):
 
 def test_lists_with_room(gbdev):
     assert _launches(gbdev, (8, 6), 0, 3, tail_from=2) == [3, 3, 3]
+
+
+def test_views_after_a_full_list(gbdev):
+    """The next sixteen views of the scene keep the node-by-node walk, then the ordered one is tried
+    again, and 32 views later; another scene starts anew."""
+    s, arrays, cam = _scene()
+    other = gbdev.RTScene(*arrays).build_bvh()
+    got = []
+    for counting in (True, False):
+        r = gbdev.RTRenderer(61, 37, 0, _params(tail_from=5))
+        r.set_counting(counting)
+        n = []
+        for k in range(53):
+            r.render(s, dict(cam, pos=(5.0, 5.0, 16.0 + 0.01 * k)))
+            n.append(r.last_stats["launches"])
+        r.render(other, cam)
+        n.append(r.last_stats["launches"])
+        got.append((n, r.read_buffer(0)))
+    extra = [b - a for a, b in zip(got[0][0], got[1][0])]
+    assert extra == [3] + 16 * [0] + [3] + 32 * [0] + [3] + 2 * [0] + [3]
+    assert_bits_equal(got[1][1], got[0][1], "image")
