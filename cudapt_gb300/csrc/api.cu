@@ -13,9 +13,9 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -220,7 +220,7 @@ struct OrderedJob {
     if (b.nodeN < 16384u) return;  // less work than starting a thread
     try {
       th = std::thread([this]() { make(); });
-    } catch (const std::system_error&) {  // no thread to be had: tree() makes it
+    } catch (const std::exception&) {  // no thread, or no memory for one: tree() makes it
     }
   }
   ~OrderedJob() {
@@ -229,7 +229,7 @@ struct OrderedJob {
   void make() {
     try {
       ok = ordered_tree(bvh, &t);
-    } catch (const std::bad_alloc&) {
+    } catch (const std::exception&) {
       ok = false;
     }
   }

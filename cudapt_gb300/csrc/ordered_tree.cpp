@@ -10,8 +10,9 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <memory>
-#include <system_error>
+#include <new>
 #include <thread>
 
 #include "gbpt_internal.h"
@@ -189,7 +190,7 @@ bool each(size_t n, uint32_t threads, const F& f) {
   for (uint32_t k = 1; k < threads && k < n; k++) {
     try {
       more.emplace_back(work);
-    } catch (const std::system_error&) {  // no thread to be had: fewer do the work
+    } catch (const std::exception&) {  // no thread, or no memory for one: fewer do the work
       break;
     }
   }
