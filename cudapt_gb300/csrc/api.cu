@@ -240,17 +240,18 @@ struct OrderedJob {
   }
 };
 
-// the ordered walk's tree, where the scene's tree allows it; leaf records are
-// copies of what the device has already
+// the ordered walk's tree, where the scene's tree and the free device memory allow
+// it (nothing needs it); leaf records are copies of what the device has already
 gbpt_status upload_ordered(gbpt_scene* s, OrderedJob& job) {
   if (!job.tree()) return GBPT_OK;
   const OrderedTree& t = job.t;
-  CK(dalloc(&s->dOrd, (size_t)t.nodeN * (kOrdNodeWords / 4)));
-  CK(dalloc(&s->dOrdLeaf, (size_t)t.leafN * (kOrdLeafWords / 4)));
-  CK(cudaMemcpy(s->dOrd, t.nodes.get(), (size_t)t.nodeN * kOrdNodeWords * 4, cudaMemcpyHostToDevice));
   uint32_t* bin = nullptr;
-  CK(dalloc(&bin, t.leafN));
-  cudaError_t e = cudaMemcpy(bin, t.leaves.get(), (size_t)t.leafN * 4, cudaMemcpyHostToDevice);
+  cudaError_t e = dalloc(&s->dOrd, (size_t)t.nodeN * (kOrdNodeWords / 4));
+  if (e == cudaSuccess) e = dalloc(&s->dOrdLeaf, (size_t)t.leafN * (kOrdLeafWords / 4));
+  if (e == cudaSuccess) e = dalloc(&bin, t.leafN);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(s->dOrd, t.nodes.get(), (size_t)t.nodeN * kOrdNodeWords * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(bin, t.leaves.get(), (size_t)t.leafN * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = launch_ord_leaves(s->dNodes, s->dTris, bin, t.leafN, s->dOrdLeaf, nullptr);
   if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   DevScene dev = s->dev;
@@ -259,13 +260,17 @@ gbpt_status upload_ordered(gbpt_scene* s, OrderedJob& job) {
   dev.ordRange = t.range;
   const bool keep = e == cudaSuccess && !walks_pass_bound(dev, bin, nullptr, &e);
   dfree(bin);
-  CK(e);
   if (keep) {
     s->dev = dev;
   } else {
     dfree(s->dOrd);
     dfree(s->dOrdLeaf);
   }
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();  // the scene does without
+    return GBPT_OK;
+  }
+  CK(e);
   return GBPT_OK;
 }
 
@@ -323,10 +328,10 @@ gbpt_status upload_scene(gbpt_scene* s) {
     gbpt_status w = upload_wide(s);
     if (w != GBPT_OK) return w;
   }
-  gbpt_status od = upload_ordered(s, ordered);
-  if (od != GBPT_OK) return od;
   gbpt_status tx = upload_textures(s);
   if (tx != GBPT_OK) return tx;
+  gbpt_status od = upload_ordered(s, ordered);  // last: it makes do with the memory that is left
+  if (od != GBPT_OK) return od;
   s->uploaded = true;
   return GBPT_OK;
 }
