@@ -469,7 +469,7 @@ def bench_gpu(args, wl):
                    "eye_depth_max": wl["depth"], "light_depth_max": wl["depth"], "tris": int(len(t)),
                    "l2": "flushed before every timed step (256 MB device memset)",
                    "bvh_build_s": round(build_s, 4), "rays_per_s": round(rays / (total_ms / 1e3), 1),
-                   "traversal": args.traversal,
+                   "traversal": "ordered" if args.traversal == "reference" else args.traversal,
                    "phase_ms_per_step": {k: round(v_ / args.steps, 4) for k, v_ in phases.items()},
                    "parallelism": "replicas" if world > 1 else "single"},
         "e2e": {"value": round(e2e * world, 3), "unit": "Mpaths/s", "h2d_bytes_per_step": 40,
@@ -551,7 +551,8 @@ def main():
     ap.add_argument("--no-extras", action="store_true", help="skip the wide walk and the other configurations")
     ap.add_argument("--no-serving", action="store_true", help="skip the batched-serving runs")
     ap.add_argument("--traversal", default="reference", choices=["reference", "wide"],
-                    help="BVH walk order: the reference's (bit-exact, default) or the collapsed 4-wide tree")
+                    help="BVH walk order: the reference's (bit-exact, by the ordered eight-wide walk; default) or "
+                         "the collapsed 4-wide tree")
     args = ap.parse_args()
     wl = dict(WORKLOADS[args.workload])
     if args.size:

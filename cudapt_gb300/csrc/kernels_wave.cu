@@ -3,7 +3,7 @@
 // One frame of the reference's streaming BDPT (src/cudaRTBDPTStream.cu:816-951)
 // runs as a fixed sequence of launches with no host round trip:
 //
-//   light pass (1 CTA)          pt_genLightPathQueue_kernel + pt_traceLight_kernel
+//   light pass                  pt_genLightPathQueue_kernel + pt_traceLight_kernel
 //                               loop with stable compaction (:875-906)
 //   camera                      pt_genPathQueue_kernel (:619-640)
 //   per bounce launch d (k_walk, then k_shade):
@@ -244,7 +244,8 @@ __device__ __forceinline__ LV load_lv(const float4* c) {
 }
 
 // ---------------------------------------------------------------------------
-// Light pass: one CTA, one thread per light subpath.  Cache slots are handed
+// Light pass: a thread per light subpath in one CTA, or eight in a cluster of
+// eight CTAs (ordered walk, up to 128 subpaths).  Cache slots are handed
 // out exactly as the reference's stable remove_if does: a surviving path's
 // position in the stream equals the number of surviving paths with a lower
 // index, i.e. an exclusive scan of the "alive" flags.
@@ -1728,7 +1729,7 @@ int g_sm = 0;
 
 // Idle lanes of a warp that trigger a refill in k_walk / k_tail (tuning
 // knob, GBPT_WALK_REFILL, 1..32; 0 when unset).  Defaults, measured on the
-// interior, hall and Cornell workloads: 8 for the reference order (4-10
+// interior, hall and Cornell workloads: 2 (with carrying; before it 8, 4-10
 // within 1%, 20 3-4% slower), 20 for the wide order (10-20 within 1%, 4 2-3%
 // slower).
 uint32_t walk_refill_env() {

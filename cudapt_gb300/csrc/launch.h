@@ -180,7 +180,7 @@ cudaError_t launch_shade(const DevScene& S, const FrameArgs& a, const RenderBuff
                          bool attach, cudaStream_t st);
 // Walks past the reference's pop bound that the frame takes as they ended
 // (checks_walks: whether it does): launch_verify checks those of the bounce
-// launches (list 0) or the tail kernel (1, after list 0), launch_tail_again
+// launches (list 0) or the tail kernel (1, after list 0), launch_again
 // runs the paths of the wrong ones again from there.
 bool checks_walks(const DevScene& S, const FrameArgs& a);
 cudaError_t launch_verify(const DevScene& S, const RenderBuffers& b, uint32_t list, cudaStream_t st);
@@ -202,7 +202,7 @@ cudaError_t launch_tail(const DevScene& S, const FrameArgs& a, const RenderBuffe
 uint32_t tail_from(uint32_t eyeDepth, bool wide, bool ordered, int32_t requested, size_t paths, bool carrying,
                    bool beside);
 // refill threshold of the persistent walks: `requested` when 1..32, else
-// GBPT_WALK_REFILL when set, else 8 (reference order) or 20 (wide order)
+// GBPT_WALK_REFILL when set, else 2, or 20 (wide order)
 uint32_t walk_refill_for(uint32_t requested, bool wide);
 // The ordered walk's leaf records (ordered.h): record k is binary leaf bin[k]
 // of `nodes` with its first triangle of `tris`.

@@ -12,14 +12,21 @@
 // sequence of triangle tests.  ordered_tree.cpp collapses the binary tree to
 // eight children a node in that order, moves every child plane outwards past
 // the rounding of both walks and stores it in 8 bits; leaf records hold the
-// exact box, tested here with the reference's arithmetic.
+// exact box, tested here with the reference's arithmetic.  Eight-wide nodes with
+// 8-bit planes on a grid of their own, and the least-cost collapse, are Ylitie,
+// Karras and Laine's ("Efficient Incoherent Ray Traversal on GPUs Through
+// Compressed Wide BVHs", HPG 2017); keeping the leaf order, and with it every
+// answer, is not.
 //
 // What is left of the reference's limits: its 2048 pops.  A pop is the root or
 // a child of an accepted inner node, and every accepted inner node lies in a
 // visited wide node, so 1 + 2 * (inner nodes of the visited wide nodes) bounds
 // the pops.  A walk whose bound passes 2048 (about 0.01 % of rays in the
 // 332,180-triangle hall) is resolved by resolve_capped(), which counts the
-// reference's pops exactly (kernels k_resolve and k_verify).
+// reference's pops exactly (kernels k_resolve and k_verify).  Scenes where that
+// happens to more than a few per mille of random rays (walks_pass_bound), and
+// scenes whose outward margin is large against their leaves (most_growth), keep
+// the node-by-node walk.
 //
 // Cost: hall rays visit 22 wide nodes and 5-7 leaves on average where the
 // binary walk pops 150-165 nodes one dependent fetch after another; a node

@@ -1,8 +1,9 @@
 // Host side of the ordered walk (ordered.cuh): the binary tree of
 // bvh_build.cpp collapsed to nodes of up to eight children that keep the order
 // in which the reference's walk reaches leaves, with child boxes in 8 bits a
-// plane, and the binary leaf of every leaf record (the device fills the records
-// in from the arrays it has: launch_ord_leaves).
+// plane (compressed wide BVHs and their least-cost collapse: Ylitie, Karras and
+// Laine, HPG 2017), and the binary leaf of every leaf record (the device fills
+// the records in from the arrays it has: launch_ord_leaves).
 //
 // Binary subtrees are index ranges, so checks and plan run over some 64 of them
 // on several threads, and so does the making of the nodes below the top ones.
