@@ -1572,9 +1572,11 @@ __global__ void k_ord_leaves(const float4* __restrict__ nodes, const float4* __r
   r[3] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(many ? first | kOrdManyTris : first));
 }
 
-// How many of n random rays inside the scene's box pass the pop bound, asked once
-// per scene.  Bound by the longest walk (146 visits reach the bound), so a warp a
-// block spreads the rays over as many SMs as there are.
+// How many of n random rays pass the pop bound, asked once per scene: every other
+// one from anywhere in the scene's box, the rest from the middle of a random
+// triangle, as most of a renderer's rays start (a model whose rays pass the bound
+// may fill little of a large space).  Bound by the longest walk (146 visits reach
+// the bound), so a warp a block spreads the rays over as many SMs as there are.
 __global__ void k_probe_walks(DevScene S, uint32_t n, uint32_t* capped) {
   using namespace gb;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1582,15 +1584,21 @@ __global__ void k_probe_walks(DevScene S, uint32_t n, uint32_t* capped) {
   const float4 lo = S.nodes[0], hi = S.nodes[1];
   float u[8];
   draw8(0u, 0u, i, 0u, kCamera, 0u, 0u, u);
-  const f3 o = mk(lo.x + (hi.x - lo.x) * u[0], lo.y + (hi.y - lo.y) * u[1], lo.z + (hi.z - lo.z) * u[2]);
   float sn, cs;
   sincos_p(kTwoPi * u[3], &sn, &cs);
   const float z = 2.f * u[4] - 1.f, q = sqrtf(1.f - z * z);
+  const f3 d = mk(q * cs, q * sn, z);
+  f3 o = mk(lo.x + (hi.x - lo.x) * u[0], lo.y + (hi.y - lo.y) * u[1], lo.z + (hi.z - lo.z) * u[2]);
+  if (i & 1u) {
+    const float4* t = S.tris + 4 * (size_t)min((uint32_t)(u[5] * (float)S.triN), S.triN - 1u);
+    const float4 p0 = t[0], e0 = t[1], e1 = t[2];
+    o = mk(p0.x + (e0.x + e1.x) / 3.f, p0.y + (e0.y + e1.y) / 3.f, p0.z + (e0.z + e1.z) / 3.f) + kBias * d;
+  }
   OrdWalk w;
   uint2 stack[kOrdStack];
   w.any = false;
   w.eps = kBias;
-  w.init(S, o, mk(q * cs, q * sn, z), kInf);
+  w.init(S, o, d, kInf);
   while (!w.capped() && !w.step(S, stack)) {
   }
   if (w.capped()) atomicAdd(capped, 1u);
@@ -1808,13 +1816,14 @@ cudaError_t launch_ord_leaves(const float4* nodes, const float4* tris, const uin
   return cudaGetLastError();
 }
 
-// Of the random rays, more than this share past the bound and the scene keeps the
+// More of the 2,048 random rays than this past the bound, and the scene keeps the
 // node-by-node walk, as resolving them costs more than the others gain.  Measured,
 // node-by-node walk / ordered (100,000 rays; 640x360 passes, each of a new view), by
-// the share of 16,384 rays: hall 0.01 % 1.69 / 1.97, hair of 40,000 strands 0.1 %
-// 1.81 / 2.39, fur of 300,000 0.16 % 1.72 / 2.45; crossing sticks 1.0 % 0.65 / 2.03,
-// 4 % 0.67 / 0.21, 20 % 0.44 / 0.17, longer hair 1.7 % 0.91 / 1.65, 6 % 0.78 / 0.76,
-// longer fur 3 % 0.87 / 1.26, 12 % 0.76 / 0.43.
+// their number: hall 0 1.69 / 1.97, finer interior 1 1.82 / 2.00, hair of 40,000
+// strands 2 1.81 / 2.39, fur of 300,000 2 1.72 / 2.45; 2,000 crossing sticks 30 0.65
+// / 2.03, longer hair 38 0.91 / 1.65, longer fur 58 0.87 / 1.26, hair 155 0.78 / 0.76,
+// sticks 190 0.67 / 0.21, fur 241 0.76 / 0.43, 6,000 sticks 920 0.44 / 0.17 and in a
+// large space 696 - / 0.16.
 constexpr uint32_t kProbeRays = 2048, kMostCapped = 10;
 
 bool walks_pass_bound(const DevScene& S, uint32_t* word, cudaStream_t st, cudaError_t* err) {

@@ -17,15 +17,20 @@ SIZES = [(61, 37), (16, 9)]  # more such walks than the lists hold, and fewer
 
 @functools.lru_cache(maxsize=None)
 def _scene():
-    """The sticks in a space so large that few of its rays meet them: it gets the ordered walk's tree."""
+    """The sticks among so many other triangles that few of the scene's rays meet them: it gets the
+    ordered walk's tree."""
     import cudapt_gb300 as gb
     (v, t, m), cam = _sticks(6000)
-    far = np.zeros(6, v.dtype)
-    far["pos"] = np.repeat(np.float32([[-150.0], [160.0]]), 3, 0) + np.tile(np.eye(3, dtype=np.float32), (2, 1))
+    n = 620  # a far floor of 2 n^2 small triangles
+    at = np.linspace(-600, 610, n + 1, dtype=np.float32)
+    x, z = np.meshgrid(at, at)
+    far = np.zeros((n + 1) ** 2, v.dtype)
+    far["pos"] = np.stack([x.ravel(), np.full(x.size, -600, np.float32), z.ravel()], 1)
     far["norm"] = (0.0, 1.0, 0.0)
-    ft = np.zeros(2, t.dtype)
-    for k, name in enumerate(("v0", "v1", "v2")):
-        ft[name] = len(v) + np.array([k, 3 + k])
+    i = (np.arange(n)[:, None] * (n + 1) + np.arange(n)).ravel() + len(v)
+    ft = np.zeros(2 * n * n, t.dtype)
+    for name, corner in (("v0", (0, 0)), ("v1", (n + 2, n + 1)), ("v2", (1, n + 2))):
+        ft[name] = np.concatenate([i + corner[0], i + corner[1]])
     v, t = np.concatenate([v, far]), np.concatenate([t, ft])
     s = gb.RTScene(v, t, m).build_bvh()
     assert (s.trace_rays(camera_rays(cam, *SIZES[0], 1), counts=True, eps=1e-4)["nodes"] == 2048).sum() > 100
@@ -46,11 +51,17 @@ def _params(**kw):
 
 
 @functools.lru_cache(maxsize=None)
+def _oracle_scene():
+    import oracle
+    return oracle.Scene(*_scene()[1])
+
+
+@functools.lru_cache(maxsize=None)
 def _want(size, mode, light_every):
     import oracle
-    _, arrays, cam = _scene()
+    cam = _scene()[2]
     ref = oracle.Renderer(*size, mode, _params(light_every=light_every))
-    ref.render(oracle.Scene(*arrays), cam, 5)
+    ref.render(_oracle_scene(), cam, 5)
     return ref.get(0), ref.sample_counts()[0]
 
 

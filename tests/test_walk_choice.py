@@ -1,6 +1,7 @@
 """A scene whose rays often run past the reference's pop bound keeps the
 node-by-node walk, others get the ordered one, seen by the three launches a frame
 of the ordered walk adds to check its answers.  Images are equal either way."""
+import numpy as np
 import pytest
 
 from helpers import assert_bits_equal, scene_arrays
@@ -9,9 +10,20 @@ from test_ordered import _sticks
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("name,ordered", [("interior", True), ("hall_small", True), ("sticks", False)])
+def _model_in_a_space():
+    """The sticks in a space so large that rays from anywhere in it hardly meet them."""
+    (v, t, m), cam = _sticks(4000)
+    far = np.zeros(6, v.dtype)
+    far["pos"] = np.repeat(np.float32([[-600.0], [610.0]]), 3, 0) + np.tile(np.eye(3, dtype=np.float32), (2, 1))
+    ft = np.zeros(2, t.dtype)
+    for k, corner in enumerate(("v0", "v1", "v2")):
+        ft[corner] = len(v) + np.array([k, 3 + k])
+    return (np.concatenate([v, far]), np.concatenate([t, ft]), m), cam
+
+
+@pytest.mark.parametrize("name,ordered", [("interior", True), ("hall_small", True), ("sticks", False), ("model", False)])
 def test_walk_of_the_scene(gbdev, name, ordered):
-    (v, t, m), cam = _sticks(4000) if name == "sticks" else scene_arrays(name)
+    (v, t, m), cam = {"sticks": lambda: _sticks(4000), "model": _model_in_a_space}.get(name, lambda: scene_arrays(name))()
     s = gbdev.RTScene(v, t, m).build_bvh()
     got = []
     for counting in (True, False):
